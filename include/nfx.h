@@ -39,12 +39,12 @@ enum {
 enum { NFX_F32 = 0, NFX_F64 = 1 };
 
 /* Threads per point of the spread / interpolation kernels (nfx_opts::spread_mode,
- * interp_mode).  AUTO: the library's choice (spread: the CTA in 3D when there are
- * fewer points than grid cells, else a warp; interpolation: a lane group in 3D,
+ * interp_mode).  AUTO: the library's choice (spread: a warp, or the CTA for wide 3D
+ * kernels with fewer points than grid cells; interpolation: a lane group in 3D,
  * one thread in 1D/2D).  THREAD: one thread per point (interpolation).  GROUP:
  * one lane group of the power of two >= nspread lanes per point, a lane per
- * footprint column (interpolation, 2D/3D).  WARP: one warp per point, a lane per
- * footprint column, runs of same-cell points summed in registers (spread).
+ * footprint column (interpolation, 2D/3D).  WARP: one warp per point, lanes
+ * over the footprint, neighbouring points summed in registers (spread).
  * CTA: every warp of the CTA on each point, a warp per tile z-plane, no atomics
  * (spread, 3D, nspread >= 4).  A mode that does not apply to a dimension falls
  * back to AUTO. */

@@ -196,14 +196,13 @@ constexpr size_t kSmemBudget = 200 * 1024;
 
 static size_t real_bytes(int precision) { return precision == NFX_F64 ? 8 : 4; }
 
-// Row pitch (cells) of the shared-memory tile.  Footprints of at least 32
-// cells in 2D/3D use the run-merging spread, whose flush has lane (grp, kx)
-// add to footprint row rho = grp * rpl + r (2D: y = rho; 3D: z = rho / ns,
-// y = rho % ns), column kx: the pitch (at most a quarter longer than the row)
-// is the one that puts those 32 words in the fewest shared-memory banks per
-// instruction.  Otherwise rows of one footprint are `ns` cells wide and a warp
-// covers 32/ns rows: a pitch that is an odd multiple of ns (mod 32) puts those
-// rows in disjoint bank ranges (at most ~12% longer).
+// Row pitch (cells) of the shared-memory tile.  2D/3D footprints of at least 32
+// cells: the pitch (at most a quarter longer than the row) that puts the 32
+// words of a warp holding 32 / ns footprint rows (lane (grp, kx): row grp * rpl
+// + r, column kx) in the fewest shared-memory banks.  Otherwise rows of one
+// footprint are `ns` cells wide and a warp covers 32/ns rows: a pitch that is an
+// odd multiple of ns (mod 32) puts those rows in disjoint bank ranges (at most
+// ~12% longer).
 static int flush_conflicts(int pitch, int plane, int ns, int dim) {
   const int G = run_groups(ns), rpl = run_rows_per_lane(dim, ns), nr = run_rows(dim, ns);
   int worst = 0;
@@ -249,6 +248,7 @@ static void fill_geom(const nfx_opts* o, Geom& g) {
     g.nb[d] = act ? (g.nf[d] + g.tile[d] - 1) / g.tile[d] : 1;
     g.pad[d] = act ? g.tile[d] + o->nspread - 1 : 1;
     g.tdiv[d] = make_fastdiv(g.tile[d]);
+    g.ndiv[d] = make_fastdiv(g.nf[d]);
   }
   g.pitch = choose_pitch(g.pad[0], g.pad[1], o->nspread, o->dim);
   g.nbins = g.nb[0] * g.nb[1] * g.nb[2];
@@ -461,6 +461,8 @@ static SortView view(const SortLayout& L, const void* ws) {
   SortView v;
   for (int d = 0; d < 3; ++d) v.coord[d] = P.coord[d];
   v.extra = P.extra;
+  v.keys = P.keys_sorted;
+  v.cbits = L.cbits;
   v.perm = P.perm;
   v.bin_start = P.bin_start;
   v.sub_bin = P.sub_bin;
@@ -661,7 +663,27 @@ static cudaError_t grad_dim(const Prepared& P, const void* x, const void* y, con
   }
 }
 
+// Shared memory of a spread launch on one problem.
+static size_t spread_launch_smem(const nfx_opts& o, const Geom& g) {
+  if (o.precision == NFX_F32)
+    return o.dim == 1   ? spread_smem_dim<float, 1>(o.nspread, g)
+           : o.dim == 2 ? spread_smem_dim<float, 2>(o.nspread, g)
+                        : spread_smem_dim<float, 3>(o.nspread, g);
+  return o.dim == 1   ? spread_smem_dim<double, 1>(o.nspread, g)
+         : o.dim == 2 ? spread_smem_dim<double, 2>(o.nspread, g)
+                      : spread_smem_dim<double, 3>(o.nspread, g);
+}
+
 static int64_t grid_cells(const Geom& g) { return (int64_t)g.nf[0] * g.nf[1] * g.nf[2]; }
+
+// Chooses the work items of one problem of a batched spread (M_total points
+// over all problems) like a plain launch.
+template <typename T>
+static int64_t split_batch_items(const Prepared& P, int64_t M_total, PointArgs<T>& a) {
+  return P.o.dim == 1   ? split_spread_items<T, 1>(P.o.nspread, M_total, a)
+         : P.o.dim == 2 ? split_spread_items<T, 2>(P.o.nspread, M_total, a)
+                        : split_spread_items<T, 3>(P.o.nspread, M_total, a);
+}
 
 template <typename T>
 __global__ void k_batch_prefix(const BatchItem<T>* __restrict__ items, int n, int* __restrict__ prefix) {
@@ -669,7 +691,7 @@ __global__ void k_batch_prefix(const BatchItem<T>* __restrict__ items, int n, in
   int run = 0;
   for (int p = 0; p < n; ++p) {
     prefix[p] = run;
-    run += *items[p].a.s.nsub;
+    run += spread_items(items[p].a);
   }
   prefix[n] = run;
 }
@@ -836,7 +858,7 @@ static int wave_layout(const nfx_opts* common, const nfx_wave_item* items, int n
     }
     if (it.kind == 1) {
       ++W.n1;
-      W.smem_s = std::max(W.smem_s, spread_smem_bytes(rb, P.o.dim, P.o.nspread, P.g));
+      W.smem_s = std::max(W.smem_s, spread_launch_smem(P.o, P.g));
       W.subs_s += P.L.max_subs;
     } else {
       ++W.n2;
@@ -868,6 +890,8 @@ static void wave_items(const nfx_opts* common, const nfx_wave_item* items, int n
   BatchItem<T>* sp = (BatchItem<T>*)(host + W.off_spread);
   BatchItem<T>* ip = (BatchItem<T>*)(host + W.off_interp);
   int a = 0, b = 0;
+  int64_t M1 = 0;
+  for (int i = 0; i < n; ++i) M1 += items[i].kind == 1 ? items[i].M : 0;
   std::vector<int> nf1, nm1, nf2, nm2;
   std::vector<const void*> fac1, fac2, src1, src2;
   std::vector<void*> dst1, dst2;
@@ -877,6 +901,7 @@ static void wave_items(const nfx_opts* common, const nfx_wave_item* items, int n
     BatchItem<T>& bi = it.kind == 1 ? sp[a++] : ip[b++];
     bi.a = make_args<T>(P.g, P.o.beta, P.o.kc, it.M, 1, view(P.L, it.workspace));
     attach_poly(bi.a, P.o.nspread, P.o.beta, P.o.kc);
+    if (it.kind == 1) split_batch_items<T>(P, M1, bi.a);
     bi.src = it.kind == 1 ? it.in : it.fw;
     bi.dst = it.kind == 1 ? it.fw : it.out;
     auto& nf = it.kind == 1 ? nf1 : nf2;
@@ -1284,7 +1309,7 @@ int nfx_batch_info_get(const nfx_opts* common, int spread, const nfx_batch_probl
     fill_geom(&P.o, P.g);
     make_layout(P.o, P.g, probs[p].M, P.L);
     const size_t rb = real_bytes(P.o.precision);
-    const size_t sm = spread ? spread_smem_bytes(rb, P.o.dim, P.o.nspread, P.g) : tile_smem_bytes(rb, P.g);
+    const size_t sm = spread ? spread_launch_smem(P.o, P.g) : tile_smem_bytes(rb, P.g);
     smem = sm > smem ? sm : smem;
     subs += P.L.max_subs;
   }
@@ -1304,6 +1329,8 @@ int nfx_batch_upload(const nfx_opts* common, int spread, const nfx_batch_problem
     return NFX_ERR_WORKSPACE;
   }
   std::vector<unsigned char> host(batch_item_bytes(common->precision) * nprob);
+  int64_t M_total = 0;
+  for (int p = 0; p < nprob; ++p) M_total += probs[p].M;
   for (int p = 0; p < nprob; ++p) {
     Prepared P;
     st = batch_problem_opts(common, probs[p], P);
@@ -1316,11 +1343,13 @@ int nfx_batch_upload(const nfx_opts* common, int spread, const nfx_batch_problem
       BatchItem<float>* it = (BatchItem<float>*)host.data() + p;
       it->a = make_args<float>(P.g, P.o.beta, P.o.kc, probs[p].M, 1, view(P.L, probs[p].workspace));
       attach_poly(it->a, P.o.nspread, P.o.beta, P.o.kc);
+      if (spread) split_batch_items<float>(P, M_total, it->a);
       it->src = probs[p].src;
       it->dst = probs[p].dst;
     } else {
       BatchItem<double>* it = (BatchItem<double>*)host.data() + p;
       it->a = make_args<double>(P.g, P.o.beta, P.o.kc, probs[p].M, 1, view(P.L, probs[p].workspace));
+      if (spread) split_batch_items<double>(P, M_total, it->a);
       it->src = probs[p].src;
       it->dst = probs[p].dst;
     }

@@ -120,6 +120,34 @@ __device__ __forceinline__ void red_add(double2* addr, double2 v) {
   atomicAdd(&addr->y, v.y);
 }
 
+// ---- block-wide exclusive scan of one int per thread ----------------------
+__device__ __forceinline__ int block_exclusive_scan(int v, int* s_warp, int& total) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  int inc = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int n = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += n;
+  }
+  if (lane == 31) s_warp[wid] = inc;
+  __syncthreads();
+  if (wid == 0) {
+    const int nw = blockDim.x >> 5;
+    int t = lane < nw ? s_warp[lane] : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int n = __shfl_up_sync(0xffffffffu, t, o);
+      if (lane >= o) t += n;
+    }
+    if (lane < nw) s_warp[lane] = t;
+  }
+  __syncthreads();
+  total = s_warp[(blockDim.x >> 5) - 1];
+  const int res = inc - v + (wid > 0 ? s_warp[wid - 1] : 0);
+  __syncthreads();
+  return res;
+}
+
 // Paired FMA: (a.x * b.x + c.x, a.y * b.y + c.y), each rounded once to
 // nearest.  float uses Blackwell's fma.rn.f32x2 (one instruction, the same
 // results as two fmaf) on 64-bit register pairs; the packing is plain C++ so
@@ -141,6 +169,40 @@ __device__ __forceinline__ double2 fma2(double2 a, double2 b, double2 c) {
   d.x = fma(a.x, b.x, c.x);
   d.y = fma(a.y, b.y, c.y);
   return d;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  unsigned long long d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(pack2(a)), "l"(pack2(b)));
+  return unpack2(d);
+}
+__device__ __forceinline__ double2 mul2(double2 a, double2 b) { return make_double2(a.x * b.x, a.y * b.y); }
+// A pair of reals as one register operand of fma2: 64 bits for float (kept
+// packed through loops, so that no moves rebuild it), a double2 for double.
+__device__ __forceinline__ unsigned long long pair_of(float a, float b) { return pack2(make_float2(a, b)); }
+__device__ __forceinline__ double2 pair_of(double a, double b) { return make_double2(a, b); }
+__device__ __forceinline__ float2 unpair(unsigned long long v) { return unpack2(v); }
+__device__ __forceinline__ double2 unpair(double2 v) { return v; }
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+template <typename T> struct PairOf;
+template <> struct PairOf<float> { using type = unsigned long long; };
+template <> struct PairOf<double> { using type = double2; };
+// red_add of a value that is not zero (predicated, no branch).
+__device__ __forceinline__ void red_add_nonzero(float2* addr, float2 v) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.neu.f32 p, %1, 0f00000000;\n setp.neu.or.f32 p, %2, 0f00000000, p;\n"
+      " @p red.global.add.v2.f32 [%0], {%1, %2};\n}" ::"l"(addr), "f"(v.x), "f"(v.y)
+      : "memory");
+}
+__device__ __forceinline__ void red_add_nonzero(double2* addr, double2 v) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.neu.f64 p, %1, 0d0000000000000000;\n"
+      " setp.neu.or.f64 p, %2, 0d0000000000000000, p;\n @p red.global.add.f64 [%0], %1;\n"
+      " @p red.global.add.f64 [%0+8], %2;\n}" ::"l"(addr), "d"(v.x), "d"(v.y)
+      : "memory");
 }
 // c + s * v for a real s and a complex v.
 __device__ __forceinline__ float2 fma_rc(float s, float2 v, float2 c) { return fma2(make_float2(s, s), v, c); }
@@ -215,6 +277,7 @@ struct Geom {
   int spread_mode;  // nfx_opts::spread_mode (threads per point of the spread)
   int interp_mode;  // nfx_opts::interp_mode (threads per point of the interpolation)
   FastDiv tdiv[3];  // division by tile[d]
+  FastDiv ndiv[3];  // division by nf[d]
   // Type 3 fused into the sort (0: off).  1: the points are type-3 sources,
   // rescaled as x' = mod((x - C) / gamma + pi, 2 pi) - pi before the fold, and
   // the sort writes each point's pre-phase e^{i isign sum_d D_d x_d};

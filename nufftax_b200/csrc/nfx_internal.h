@@ -61,6 +61,8 @@ struct SortView {
   // the spread multiplies into the strength (sources: the pre-phase) or the
   // interpolation into the value it writes (targets: phase / phihat).
   const void* extra;
+  const int* keys;  // composite keys in sorted order: bin << cbits | cell
+  int cbits;
   const int* perm;
   const int* bin_start;
   const int* sub_bin;
@@ -139,16 +141,12 @@ int* device_status_word();
 // Warps per CTA of the spread / interp / gradient kernels.
 constexpr int warps_per_cta(size_t real_bytes, int dim, int ns) { return (real_bytes == 8 && dim == 3) ? 4 : 8; }
 
-// Run-merging spread layout (2D/3D footprints of at least 32 cells): lane l of
-// a warp owns footprint column kx = l % ns and rows (y, or z*ns + y) grp*rpl ..
-// grp*rpl + rpl - 1 with grp = l / ns; the 32 / ns groups cover the ns^(dim-1)
-// rows.  A staged point is one slot of reals: c * w_x (ns complex), then the y
-// weights and (3D) the z weights.  Sections are padded to the rows the groups
-// reach and to whole 16-byte chunks; the slot length (4 mod 8 floats, 2 mod 4
-// doubles) makes the 16-byte stores of a warp (one slot per lane) hit distinct
-// banks.  The walk reads the weights with scalar loads: every lane of a group
-// reads the same word (one broadcast wavefront), which keeps the shared-memory
-// pipe less busy than wider loads would.
+// Slot layout (2D/3D footprints of at least 32 cells) that the shared-memory
+// budget of a tile counts per staged point: c * w_x (ns complex), then the y
+// weights and (3D) the z weights, padded to the 32 / ns row groups a warp covers
+// and to whole 16-byte chunks.  The window spread's own slots are no larger in
+// total; the budget keeps this form so that the default tiles, and the tiles
+// that are refused, stay what they are.
 // run_slot_reals is 0 when the layout does not apply (1D, small footprints,
 // more than 16 rows a lane).
 __host__ __device__ constexpr int run_groups(int ns) { return 32 / ns; }
@@ -174,9 +172,9 @@ __host__ __device__ constexpr int run_slot_reals(int dim, int ns, int real_bytes
              : 0;
 }
 
-// Dynamic shared memory of the spread kernel: two planar tile planes plus the
-// per-warp staging of 32 points (weights, strengths; tile offsets for the
-// layout without run merging).
+// Dynamic shared memory of the tile spread: two planar tile planes plus the
+// per-warp staging of 32 points (weights, strengths, tile offsets); also the
+// budget that the tile edges are chosen by (for every kernel).
 inline size_t spread_smem_bytes(size_t real_bytes, int dim, int ns, const Geom& g) {
   const int nw = warps_per_cta(real_bytes, dim, ns);
   const size_t tile = 2 * real_bytes * (size_t)g.pad[2] * g.pad[1] * g.pitch;

@@ -78,35 +78,6 @@ __device__ __forceinline__ void cell_keys(const T (&c)[DIM], const Geom& g, int 
   kcell = kc;
 }
 
-// ---- block-wide exclusive scan of one int per thread ----------------------
-__device__ __forceinline__ int block_exclusive_scan(int v, int* s_warp, int& total) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  int inc = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int n = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= o) inc += n;
-  }
-  if (lane == 31) s_warp[wid] = inc;
-  __syncthreads();
-  if (wid == 0) {
-    const int nw = blockDim.x >> 5;
-    int t = lane < nw ? s_warp[lane] : 0;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int n = __shfl_up_sync(0xffffffffu, t, o);
-      if (lane >= o) t += n;
-    }
-    if (lane < nw) s_warp[lane] = t;
-  }
-  __syncthreads();
-  total = s_warp[(blockDim.x >> 5) - 1];
-  const int res = inc - v + (wid > 0 ? s_warp[wid - 1] : 0);
-  __syncthreads();
-  return res;
-}
-
-
 constexpr int kRadixThreads = 256;
 constexpr int kRadixItems = 16;
 constexpr int kRadixChunk = kRadixThreads * kRadixItems;  // elements per chunk (one CTA)

@@ -1,0 +1,540 @@
+// Register-window spreading (2D, and 3D for the widths whose windows fit in
+// registers).
+//
+// A warp takes the points whose left cells lie in one small block (BX x BY [x BZ]
+// cells) and keeps the whole window those footprints cover (NS + B - 1 cells per
+// axis) in its registers: every point adds (c w_x) w_y [w_z] to all of the
+// window's cells, with zero weights outside its own footprint, so the inner loop
+// has no address, no branch and no shared-memory update per cell.  When the
+// block changes the window goes straight to the fine grid with vectorised reds,
+// lanes along x.
+//
+// Why: a spread that adds every footprint cell to a shared-memory tile is bound
+// by that update (a float add on shared memory is a compare-and-swap loop here,
+// a plain read-add-write 64 of the 107 shared wavefronts a 3D point cost at
+// ns = 8) while the FMA pipe idles.  Reds of windows to L2 run at 590 G complex64
+// cells/s when the blocks follow the bin order (4x4x4 windows of a 256^3 grid,
+// 348 M cells in 594 us; a CTA tile flushed by compare-and-swap takes as long)
+// and are fire-and-forget, and the window sums the block's points first: at 0.5
+// points per cell a 3D point costs 43 reds instead of 512 updates.
+//
+// Block shapes.  3D: 4x4x4 cells for complex64 (window 11^3 at ns = 8: 44 paired
+// FMAs a lane and point, 17 ns per point and SM alone; 4x4x2 needs 36 but 1.6
+// times the reds), 2x2x2 for complex128 (accumulators of twice the registers).
+// A 3D block's points are not contiguous in the sorted order (cells x-fastest),
+// so each CTA first groups its item's points by block with a counting sort of
+// 16-bit indices in shared memory (two passes over the sorted keys).  2D
+// complex64: segments of 8x1 cells, which are contiguous, so nothing is grouped
+// (8x4 blocks measured 227 us instead of 146 on 4M clustered points: grouping
+// and the wider window cost more than the reds they save).  2D complex128:
+// blocks, since a wide kernel's window is all reds.
+//
+// What bounds it now (sorted points, L2 flushed before each call; before = the
+// shared-memory tile spreads it replaces): 3D 8M points on 256^3, ns 8: 3645 ->
+// 1725 us (FMA pipe 51 %, issue 54 %); 1M on 192x225x256: 781 -> 505 us (reds,
+// L2 57 %); 2D 524 k radial on 1024^2, ns 8: 91 -> 52 us, 4M clustered 163 -> 146
+// us (staging: issue 63 %, shared memory 87 %); 2D complex128 ns 14, 200 k
+// points: 412 -> 97 us (the ES weights).
+#pragma once
+
+#include <type_traits>
+
+#include "nfx_internal.h"
+
+namespace nfx {
+
+constexpr int kWinRound = 2048;   // most points of a work item (16-bit list entries)
+constexpr int kWinBlocks = 1024;  // most blocks (of all its bins) an item is grouped by
+
+// Block and lane layout per dimension and width.  2D: lane = (x, row group),
+// LW x positions times H row groups of RL rows each.  3D: a lane owns NCOL
+// (x, y) columns of WZ cells.
+template <typename T, int DIM, int NS>
+struct WinShape;
+
+template <typename T, int NS>
+struct WinShape<T, 2, NS> {
+  static constexpr bool on = true;
+  // complex64: row segments of BX cells, contiguous in the sorted order, so no
+  // grouping; complex128: BX x BY blocks (wide kernels, costly window reds)
+  static constexpr bool GROUP = sizeof(T) == 8;
+  static constexpr int LW = 16;
+  static constexpr int H = 32 / LW;
+  static constexpr int BX = NS <= 8 ? 8 : (NS <= 12 ? 4 : (NS == 14 ? 2 : 1));
+  static constexpr int BY = GROUP ? 4 : 1;
+  static constexpr int BZ = 1;
+  static constexpr int WX = NS + BX - 1, WY = NS + BY - 1;
+  static constexpr int RL = (WY + H - 1) / H;
+  static_assert(WX <= LW, "the window's x extent fits the lanes");
+  // slot: c * w_x per x position, then the row weights, both zero outside the
+  // footprint; an odd number of 16-byte units, so that slots of consecutive
+  // points start in different banks
+  static constexpr int YO = 2 * LW;
+  static constexpr int R16 = 16 / (int)sizeof(T);
+  static constexpr int RS = (RL + R16 - 1) / R16 * R16;  // a row group's weights, whole 16-byte units
+  static constexpr int YN = H * RS;
+  static constexpr int RAW = (YO + YN) / R16;
+  static constexpr int SLOT = (RAW % 2 == 0 ? RAW + 1 : RAW) * R16;
+};
+
+// Whether a (type, width) has a 3D window: NCOL * WZ complex accumulators a lane.
+template <typename T, int NS>
+struct WinShape<T, 3, NS> {
+  static constexpr bool on = NS <= 8;
+  static constexpr bool GROUP = true;
+  static constexpr int B = sizeof(T) == 4 ? 4 : 2;
+  static constexpr int BX = B, BY = B, BZ = B;
+  static constexpr int WX = NS + BX - 1, WY = NS + BY - 1, WZ = NS + BZ - 1;
+  static constexpr int NC = WX * WY;
+  static constexpr int NCOL = (NC + 31) / 32;
+  // slot: w_z, c * w_x (complex), w_y
+  static constexpr int R16 = 16 / (int)sizeof(T);
+  static constexpr int ZN = (WZ + R16 - 1) / R16 * R16;
+  static constexpr int XO = ZN;
+  static constexpr int XN = (2 * WX + R16 - 1) / R16 * R16;
+  static constexpr int YO = XO + XN;
+  static constexpr int YN = (WY + R16 - 1) / R16 * R16;
+  static constexpr int RAW = (YO + YN) / R16;
+  static constexpr int SLOT = (RAW % 2 == 0 ? RAW + 1 : RAW) * R16;
+};
+
+template <typename T, int NS>
+struct WinShape<T, 1, NS> {
+  static constexpr bool on = false;
+};
+
+// Warps per CTA of the spread (the window of 44 complex64 cells a lane needs
+// about 160 registers to run without spills).
+template <typename T, int DIM, int NS>
+constexpr int win_warps() {
+  return sizeof(T) == 4 && DIM == 3 && NS == 8 ? 6 : warps_per_cta(sizeof(T), DIM, NS);
+}
+
+// Shared memory of a window spread: the warps' slots, a count per block and
+// the block-ordered list.
+template <typename T, int DIM, int NS>
+size_t win_smem_bytes() {
+  return (size_t)win_warps<T, DIM, NS>() * 32 * WinShape<T, DIM, NS>::SLOT * sizeof(T) +
+         (WinShape<T, DIM, NS>::GROUP ? kWinBlocks * sizeof(int) + kWinRound * sizeof(unsigned short) : 0);
+}
+
+// Points of one work item of a spread of M points on `ctas` resident CTAs: the
+// items are equal, so as many as the CTAs take in whole rounds, of at most
+// kWinRound points (2D: 1024; 4M clustered points 146 us, 159 with 2048, whose
+// four rounds end unevenly).  The least size bounds the partial sums a crowded
+// cell gets (each slice of a warp adds its own, and their float rounding): 100 k
+// points in one 2D cell have a relative error of 2.5e-6 with 64-point items,
+// 1.5e-6 with 256, 0.9e-6 with 512 and no less with more.  3D points cost several
+// times a 2D point and spread over more cells, so their items may be smaller;
+// sets too small to give every SM an item of the least size are cut down to 64.
+inline int win_part_points(int dim, int64_t M, int ctas) {
+  const int64_t most = dim == 2 ? 1024 : kWinRound;
+  const int64_t least = M < 256 * 148 ? 64 : (dim == 2 ? 512 : 128);
+  const int64_t rounds = (M + ctas * most - 1) / (ctas * most);
+  const int64_t n = rounds > 0 ? (M + ctas * rounds - 1) / (ctas * rounds) : 1;
+  return (int)((n < least ? least : n) + 31) / 32 * 32;
+}
+
+// Adds one point whose strength or coordinates are not finite cell by cell
+// (its window would turn zero weights of other cells into NaN): rare, so one
+// lane loops over the footprint.
+template <typename T, int DIM, int NS>
+__device__ __forceinline__ void win_add_direct(const PointArgs<T>& a, cplx_t<T> cv, T x, T y, T z,
+                                               cplx_t<T>* __restrict__ out) {
+  const Geom& g = a.g;
+  const int ix = left_cell<T, NS>(x), iy = left_cell<T, NS>(y), iz = DIM == 3 ? left_cell<T, NS>(z) : 0;
+#pragma unroll 1
+  for (int q = 0; q < (DIM == 3 ? NS * NS * NS : NS * NS); ++q) {
+    const int kx = q % NS, ky = (q / NS) % NS, kz = q / (NS * NS);
+    T w = es_weight(rn_sub((T)(ix + kx), x), a.beta, a.kc) * es_weight(rn_sub((T)(iy + ky), y), a.beta, a.kc);
+    if (DIM == 3) w *= es_weight(rn_sub((T)(iz + kz), z), a.beta, a.kc);
+    cplx_t<T> v;
+    v.x = w * cv.x;
+    v.y = w * cv.y;
+    const int gx = wrap_index(ix + kx, g.nf[0]), gy = wrap_index(iy + ky, g.nf[1]);
+    const int gz = DIM == 3 ? wrap_index(iz + kz, g.nf[2]) : 0;
+    red_add(out + ((int64_t)gz * g.nf[1] + gy) * g.nf[0] + gx, v);
+  }
+}
+
+// i >= 0 wrapped into axis d of the grid (no branch; windows may be wider than a tiny grid).
+__device__ __forceinline__ int wrap_mod(int i, int d, const Geom& g) {
+  return i - fast_div(i, g.ndiv[d]) * g.nf[d];
+}
+
+template <typename T>
+__device__ __forceinline__ bool is_finite(T v) {
+  return v - v == (T)0;
+}
+
+template <typename T>
+__device__ __forceinline__ void zero_pair(cplx_t<T>& v) {
+  v.x = v.y = (T)0;
+}
+
+// A slot section of N reals (a multiple of 16 bytes, 16-byte aligned): zeros,
+// then NS weights from dl on (times the strength for the complex section).
+template <int N, typename T>
+__device__ __forceinline__ void stage_zero(T* s) {
+  constexpr int R = 16 / (int)sizeof(T);
+  static_assert(N % R == 0, "whole 16-byte units");
+#pragma unroll
+  for (int i = 0; i < N / R; ++i) reinterpret_cast<float4*>(s)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+}
+template <int NS, int N, typename T>
+__device__ __forceinline__ void stage_cw(T* s, cplx_t<T> cv, const T (&w)[NS], int dl) {
+  stage_zero<N>(s);
+#pragma unroll
+  for (int q = 0; q < NS; ++q) reinterpret_cast<cplx_t<T>*>(s)[dl + q] = mul2(splat2(w[q]), cv);
+}
+template <int NS, int N, typename T>
+__device__ __forceinline__ void stage_w(T* s, const T (&w)[NS], int dl) {
+  stage_zero<N>(s);
+#pragma unroll
+  for (int q = 0; q < NS; ++q) s[dl + q] = w[q];
+}
+
+// The window accumulators of one lane: add(slot) takes a staged point,
+// flush() sends the window to the grid and clears it.
+template <typename T, int DIM, int NS>
+struct Window;
+
+// acc[k] += z[k] * v[k] for the first N of the reals at zs (16-byte loads; a
+// real times a complex is one paired FMA, the real used for both halves).
+template <int N, typename T, typename F>
+__device__ __forceinline__ void for_weights(const T* zs, F f) {
+  using V16 = typename Vec16<T>::type;
+  constexpr int R = 16 / (int)sizeof(T);
+#pragma unroll
+  for (int k = 0; k < N; k += R) {
+    const V16 z = *reinterpret_cast<const V16*>(zs + k);
+    f(k, z.x);
+    if (k + 1 < N) f(k + 1, z.y);
+    if constexpr (R == 4) {
+      if (k + 2 < N) f(k + 2, z.z);
+      if (k + 3 < N) f(k + 3, z.w);
+    }
+  }
+}
+
+template <typename T, int NS>
+struct Window<T, 2, NS> {
+  using CT = cplx_t<T>;
+  using PT = typename PairOf<T>::type;
+  using W = WinShape<T, 2, NS>;
+  PT acc[W::RL];  // complex cells of this lane's rows
+  int xo, yo;     // this lane's entries of a slot
+
+  __device__ __forceinline__ explicit Window(int lane) {
+    xo = 2 * (lane % W::LW);
+    yo = W::YO + (lane / W::LW) * W::RS;
+    clear();
+  }
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int i = 0; i < W::RL; ++i) acc[i] = pair_of((T)0, (T)0);
+  }
+  // Axis D's weights (times the strength on x) at offset dl of its section,
+  // zeros in the rest of it.
+  template <int D>
+  static __device__ __forceinline__ void stage(T* sp, CT cv, const T (&w)[NS], int dl) {
+    if constexpr (D == 0) {
+      stage_cw<NS, W::YO>(sp, cv, w, dl);
+    } else {
+      stage_zero<W::YN>(sp + W::YO);
+#pragma unroll
+      for (int q = 0; q < NS; ++q) {
+        const int row = dl + q;  // row group row / RL starts at a multiple of RS
+        sp[W::YO + row + (W::RS != W::RL && row >= W::RL ? W::RS - W::RL : 0)] = w[q];
+      }
+    }
+  }
+  __device__ __forceinline__ void add(const T* sp) {
+    const PT cw = *reinterpret_cast<const PT*>(sp + xo);
+    for_weights<W::RL>(sp + yo, [&](int r, T w) { acc[r] = fma2(pair_of(w, w), cw, acc[r]); });
+  }
+  // (ox, oy, oz): the window's first cell per axis (inside the grid)
+  __device__ __forceinline__ void flush(const Geom& g, int ox, int oy, int, int lane, CT* __restrict__ out) {
+    const int x = lane % W::LW;
+    const int row0 = (lane / W::LW) * W::RL;
+    if (x < W::WX) {
+      int gy = wrap_mod(oy + row0, 1, g);
+      int at = gy * g.nf[0] + wrap_mod(ox + x, 0, g);  // grids have fewer than 2^31 cells
+#pragma unroll
+      for (int r = 0; r < W::RL; ++r) {
+        // no test for zero: skipping a red costs more than most zeros' reds
+        if ((W::H - 1) * W::RL + r < W::WY || row0 + r < W::WY) red_add(out + at, unpair(acc[r]));
+        at += g.nf[0];
+        if (++gy == g.nf[1]) {
+          gy = 0;
+          at -= g.nf[0] * g.nf[1];
+        }
+      }
+    }
+    clear();
+  }
+};
+
+template <typename T, int NS>
+struct Window<T, 3, NS> {
+  using CT = cplx_t<T>;
+  using PT = typename PairOf<T>::type;
+  using W = WinShape<T, 3, NS>;
+  PT acc[W::NCOL][W::WZ];      // complex cells
+  int xo[W::NCOL], yo[W::NCOL];  // this lane's columns' entries of a slot
+
+  __device__ __forceinline__ explicit Window(int lane) {
+#pragma unroll
+    for (int i = 0; i < W::NCOL; ++i) {
+      const int c = lane + 32 * i < W::NC ? lane + 32 * i : 0;
+      xo[i] = W::XO + 2 * (c % W::WX);
+      yo[i] = W::YO + c / W::WX;
+    }
+    clear();
+  }
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int i = 0; i < W::NCOL; ++i)
+#pragma unroll
+      for (int k = 0; k < W::WZ; ++k) acc[i][k] = pair_of((T)0, (T)0);
+  }
+  template <int D>
+  static __device__ __forceinline__ void stage(T* sp, CT cv, const T (&w)[NS], int dl) {
+    if constexpr (D == 0) {
+      stage_cw<NS, W::XN>(sp + W::XO, cv, w, dl);
+    } else if constexpr (D == 1) {
+      stage_w<NS, W::YN>(sp + W::YO, w, dl);
+    } else {
+      stage_w<NS, W::ZN>(sp, w, dl);
+    }
+  }
+  __device__ __forceinline__ void add(const T* sp) {
+    PT v[W::NCOL];
+#pragma unroll
+    for (int i = 0; i < W::NCOL; ++i) {
+      const CT cw = *reinterpret_cast<const CT*>(sp + xo[i]);
+      const T wy = sp[yo[i]];
+      v[i] = pair_of(cw.x * wy, cw.y * wy);
+    }
+    for_weights<W::WZ>(sp, [&](int k, T z) {
+      const PT zd = pair_of(z, z);
+#pragma unroll
+      for (int i = 0; i < W::NCOL; ++i) acc[i][k] = fma2(zd, v[i], acc[i][k]);
+    });
+  }
+  __device__ __forceinline__ void flush(const Geom& g, int ox, int oy, int oz, int lane, CT* __restrict__ out) {
+    const int plane = g.nf[0] * g.nf[1];  // grids have fewer than 2^31 cells
+    int at[W::NCOL];
+#pragma unroll
+    for (int i = 0; i < W::NCOL; ++i) {
+      const int c = lane + 32 * i;
+      at[i] = (oz * g.nf[1] + wrap_mod(oy + c / W::WX, 1, g)) * g.nf[0] + wrap_mod(ox + c % W::WX, 0, g);
+    }
+    const bool last_on = W::NC % 32 == 0 || lane + 32 * (W::NCOL - 1) < W::NC;  // this lane has a last column
+    int gz = oz;  // a block starts inside the grid
+#pragma unroll
+    for (int k = 0; k < W::WZ; ++k) {
+      // no test for zero: skipping a red costs more than most zeros' reds
+#pragma unroll
+      for (int i = 0; i < W::NCOL - 1; ++i) red_add(out + at[i], unpair(acc[i][k]));
+      if (last_on) red_add(out + at[W::NCOL - 1], unpair(acc[W::NCOL - 1][k]));
+      int step = plane;
+      if (++gz == g.nf[2]) {
+        gz = 0;
+        step = plane - plane * g.nf[2];
+      }
+#pragma unroll
+      for (int i = 0; i < W::NCOL; ++i) at[i] += step;
+    }
+    clear();
+  }
+};
+
+// One work item: `a.win_part` consecutive points of the sorted order (of one
+// or several bins).  The CTA groups them by block, then every warp takes a
+// contiguous slice of the grouped list 32 points at a time: each lane stages
+// one point, and the warp adds the 32 one after another, flushing the window
+// whenever the block changes.  The next 32 points are fetched while the
+// current ones are added.
+template <typename T, int DIM, int NS, int NW>
+__device__ __forceinline__ void spread_window(const PointArgs<T>& a, const cplx_t<T>* __restrict__ c,
+                                              cplx_t<T>* __restrict__ fw, int item, unsigned char* smem_raw) {
+  using CT = cplx_t<T>;
+  using W = WinShape<T, DIM, NS>;
+  constexpr int NT = NW * 32;
+  constexpr int PER = (kWinRound + NT - 1) / NT;  // most points of an item per thread
+  __shared__ int s_warp[32];
+  const Geom& g = a.g;
+  const int k0 = item * a.win_part;
+  const int n = (int)min((int64_t)a.win_part, a.M - k0);
+  T* s_slots = reinterpret_cast<T*>(smem_raw);
+  int* s_cnt = reinterpret_cast<int*>(s_slots + NT * W::SLOT);  // per block: points, then its list start
+  unsigned short* s_list = reinterpret_cast<unsigned short*>(s_cnt + kWinBlocks);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  T* my_slot = s_slots + (warp * 32 + lane) * W::SLOT;
+  const T* warp_slots = s_slots + warp * 32 * W::SLOT;
+  // ---- group the points by block: bins in order, blocks within a bin ----
+  if constexpr (W::GROUP) {
+    const int nbx = (g.tile[0] + W::BX - 1) / W::BX, nby = (g.tile[1] + W::BY - 1) / W::BY;
+    const int nbz = (g.tile[2] + W::BZ - 1) / W::BZ;
+    const int bin0 = a.s.keys[k0] >> a.s.cbits;
+    const int64_t span = (int64_t)((a.s.keys[k0 + n - 1] >> a.s.cbits) - bin0 + 1) * (nbx * nby * nbz);
+    if (span > kWinBlocks || span < 1) {
+      // few points per bin: no two of them are likely to share a block
+      for (int i = threadIdx.x; i < n; i += NT) s_list[i] = (unsigned short)i;
+    } else {
+      const int nblk = (int)span;
+      const int cmask = (1 << a.s.cbits) - 1;
+      for (int i = threadIdx.x; i < nblk; i += NT) s_cnt[i] = 0;
+      int key[PER], rank[PER];
+#pragma unroll
+      for (int i = 0; i < PER; ++i) {
+        const int j = i * NT + threadIdx.x;
+        key[i] = j < n ? a.s.keys[k0 + j] : -1;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < PER; ++i) {
+        if (key[i] >= 0) {
+          const int cell = key[i] & cmask;
+          const int r = fast_div(cell, g.tdiv[0]);
+          const int cx = cell - r * g.tile[0];
+          int blk = (key[i] >> a.s.cbits) - bin0;
+          if (DIM == 2) {
+            blk = (blk * nby + r / W::BY) * nbx + cx / W::BX;
+          } else {
+            const int cz = fast_div(r, g.tdiv[1]);
+            const int cy = r - cz * g.tile[1];
+            blk = ((blk * nbz + cz / W::BZ) * nby + cy / W::BY) * nbx + cx / W::BX;
+          }
+          key[i] = min(max(blk, 0), nblk - 1);  // keys of a sound sort are in range
+          rank[i] = atomicAdd(&s_cnt[key[i]], 1);
+        }
+      }
+      __syncthreads();
+      const int per = (nblk + NT - 1) / NT;
+      const int i0 = min((int)threadIdx.x * per, nblk), i1 = min(i0 + per, nblk);
+      int sum = 0, total;
+      for (int i = i0; i < i1; ++i) sum += s_cnt[i];
+      int run = block_exclusive_scan(sum, s_warp, total);
+      for (int i = i0; i < i1; ++i) {
+        const int v = s_cnt[i];
+        s_cnt[i] = run;
+        run += v;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < PER; ++i)
+        if (key[i] >= 0) s_list[s_cnt[key[i]] + rank[i]] = (unsigned short)(i * NT + threadIdx.x);
+    }
+    __syncthreads();
+  }
+  // ---- the warp's slice of the list, per transform ----
+  auto list_at = [&](int i) { return W::GROUP ? (int)s_list[i] : i; };
+  const int p0 = (int)((unsigned)n * warp / NW);  // slices differ by at most one point
+  const int p1 = (int)((unsigned)n * (warp + 1) / NW);
+  if (p0 < p1) {
+    Window<T, DIM, NS> win(lane);
+    for (int t = 0; t < a.n_trans; ++t) {
+      const CT* ct = c + (int64_t)t * a.M;
+      CT* const out = fw + (int64_t)t * a.grid_stride;
+      // this lane's point of the next 32 (kn < 0: none), two list entries ahead
+      T xn[DIM];
+      CT cn;
+      zero_pair<T>(cn);
+#pragma unroll
+      for (int d = 0; d < DIM; ++d) xn[d] = (T)0;
+      int kn = p0 + lane < p1 ? k0 + list_at(p0 + lane) : -1;
+      if (kn >= 0) {
+        load_sorted<T, DIM>(a, kn, xn);
+        cn = ct[a.s.perm[kn]];
+      }
+      int k2 = p0 + 32 + lane < p1 ? k0 + list_at(p0 + 32 + lane) : -1;
+      int pn = k2 >= 0 ? a.s.perm[k2] : 0;
+      int cur[3] = {-1, -1, -1};  // the open window's first cell per axis, -1: none
+      for (int p = p0; p < p1 + 32; p += 32) {
+        const int cnt = min(32, p1 - p);  // <= 0 on the last trip, which only flushes
+        const int k = kn;
+        T xv[DIM];
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) xv[d] = xn[d];
+        CT cv = cn;
+        kn = k2;
+        if (kn >= 0) {
+          load_sorted<T, DIM>(a, kn, xn);
+          cn = ct[pn];
+        }
+        k2 = p + 64 + lane < p1 ? k0 + list_at(p + 64 + lane) : -1;
+        pn = k2 >= 0 ? a.s.perm[k2] : 0;
+        // stage this lane's point, axis by axis (points added directly stage zeros)
+        int base[3] = {-1, -1, -1};
+        if (cnt > 0) {
+          int i0[DIM], dl[DIM];
+          bool fin = true;
+#pragma unroll
+          for (int d = 0; d < DIM; ++d) {
+            constexpr int kB[3] = {W::BX, W::BY, W::BZ};
+            i0[d] = left_cell<T, NS>(xv[d]);
+            const int l = wrap_index(i0[d], g.nf[d]);
+            base[d] = (int)((unsigned)l / kB[d]) * kB[d];
+            dl[d] = l - base[d];
+            fin = fin && is_finite(xv[d]);
+          }
+          if (k >= 0) cv = with_extra(a, k, cv);
+          fin = fin && is_finite(cv.x) && is_finite(cv.y);
+          if (k >= 0 && !fin) win_add_direct<T, DIM, NS>(a, cv, xv[0], xv[1], xv[DIM - 1], out);
+          if (k < 0 || !fin) {
+            zero_pair<T>(cv);
+#pragma unroll
+            for (int d = 0; d < DIM; ++d) {
+              dl[d] = i0[d] = 0;
+              xv[d] = (T)(NS / 2);
+            }
+          }
+          T w[NS];
+          axis_weights<T, NS>(a, i0[0], xv[0], w);
+          Window<T, DIM, NS>::template stage<0>(my_slot, cv, w, dl[0]);
+          axis_weights<T, NS>(a, i0[1], xv[1], w);
+          Window<T, DIM, NS>::template stage<1>(my_slot, cv, w, dl[1]);
+          if constexpr (DIM == 3) {
+            axis_weights<T, NS>(a, i0[2], xv[2], w);
+            Window<T, DIM, NS>::template stage<2>(my_slot, cv, w, dl[2]);
+          }
+        }
+        // lane j starts a block when its block differs from point j - 1's
+        bool differs = false;
+#pragma unroll
+        for (int d = 0; d < DIM; ++d) {
+          int prev = __shfl_up_sync(0xffffffffu, base[d], 1);
+          if (lane == 0) prev = cur[d];
+          differs = differs || prev != base[d];
+        }
+        const unsigned starts = cnt > 0 ? __ballot_sync(0xffffffffu, differs && lane < cnt) : 1u;
+        __syncwarp();
+        int j = 0;
+        do {  // one block (or the rest of one) per trip
+          if ((starts >> j) & 1u) {
+            if (cur[0] >= 0) win.flush(g, cur[0], cur[1], cur[2], lane, out);
+#pragma unroll
+            for (int d = 0; d < DIM; ++d) cur[d] = __shfl_sync(0xffffffffu, base[d], j);
+            if (DIM == 2) cur[2] = 0;
+          }
+          const unsigned later = j < 31 ? starts >> (j + 1) : 0u;
+          const int je = later != 0u ? min(j + __ffs(later), cnt) : cnt;
+          const T* sp = warp_slots + j * W::SLOT;
+          constexpr int U = DIM == 2 ? 4 : 2;
+          for (; j + U <= je; j += U, sp += U * W::SLOT) {
+#pragma unroll
+            for (int q = 0; q < U; ++q) win.add(sp + q * W::SLOT);
+          }
+#pragma unroll 1
+          for (; j < je; ++j, sp += W::SLOT) win.add(sp);
+        } while (j < cnt);
+        __syncwarp();
+      }
+    }
+  }
+  if constexpr (W::GROUP) __syncthreads();  // the list and counts are free for the next item
+}
+
+}  // namespace nfx

@@ -6,16 +6,14 @@
 // fine grid), so each CTA works entirely in shared memory:
 //
 //  * spread (nufftax/core/spread.py:285-339, 435-494, 596-658; Pallas twin
-//    nufftax/core/pallas_spread.py:337-613): points are staged 32 at a time per
-//    warp (each lane folds one point and evaluates its d*ns ES weights once);
-//    the warp then walks the 32 footprints one after another.  For 2D/3D
-//    footprints of at least 32 cells each lane owns one footprint column and a
-//    block of rows and sums consecutive same-cell points in registers
-//    (spread_subproblem_runs); smaller footprints go cell by cell with
-//    shared-memory atomics (spread_subproblem_cells).  Every shared-memory
-//    atomic of one instruction hits a distinct address, so clustered points do
-//    not serialise.  The finished tile is flushed with one vectorised
-//    `red.global.add.v2.f32` per non-zero cell, coalesced along x.
+//    nufftax/core/pallas_spread.py:337-613): 2D, and 3D widths up to 8, sum the
+//    window of a block of neighbouring points in a warp's registers and send it
+//    to the grid (nfx_spread_window.cuh).  The rest goes through a shared-memory
+//    tile: cell by cell with shared-memory atomics on distinct addresses
+//    (spread_subproblem_cells: 1D, and 3D of width 10 and more with points
+//    denser than cells), or plane by plane without atomics
+//    (spread_subproblem_owner: sparse 3D).  A finished tile is flushed with one
+//    vectorised `red.global.add.v2.f32` per non-zero cell, coalesced along x.
 //  * interp (nufftax/core/spread.py:342-381, 497-540, 661-709): the padded tile
 //    is staged into shared memory with coalesced loads, then each thread
 //    evaluates one point as a separable sum (x innermost); no atomics.
@@ -25,6 +23,7 @@
 #pragma once
 
 
+#include <algorithm>
 #include <type_traits>
 
 #include "nfx_internal.h"
@@ -46,6 +45,7 @@ struct PointArgs {
   int64_t M;
   int n_trans;
   int64_t grid_stride;  // complex elements per transform of the fine grid
+  int win_part;         // window spread: points of one work item; 0: an item is a subproblem
   int tma;              // 1: the interpolation stages interior tiles with the kernel's tensor map
   int* status;          // device status word (nonzero after a bounded wait gave up); set when tma = 1
   Geom g;
@@ -199,316 +199,23 @@ __device__ __forceinline__ bool point_footprint(const PointArgs<T>& a, int k, co
   return footprint<T, DIM, NS>(a, xf, o, row, plane, off, w);
 }
 
-// Slot helpers of the run-merging spread: 16-byte chunks of four floats or two
-// doubles (slots are 16-byte aligned, see run_slot_reals).
-__device__ __forceinline__ void store16(float* p, float a, float b, float c, float d) {
-  *reinterpret_cast<float4*>(p) = make_float4(a, b, c, d);
-}
-__device__ __forceinline__ void store16(double* p, double a, double b) {
-  *reinterpret_cast<double2*>(p) = make_double2(a, b);
-}
+// A 16-byte vector of T.
+template <typename T>
+struct Vec16;
+template <>
+struct Vec16<float> {
+  using type = float4;
+};
+template <>
+struct Vec16<double> {
+  using type = double2;
+};
 
-// Writes one point's slot: c * w_x, then the y weights and (3D) the z
-// weights; padding entries are zero.
-template <typename T, int DIM, int NS>
-__device__ __forceinline__ void stage_slot(T* sp, cplx_t<T> cv, const T (&w)[DIM][NS]) {
-  constexpr int WY = run_wy(DIM, NS);
-  constexpr int WZ = run_wz(DIM, NS);
-  constexpr int YOFF = round4(2 * NS);
-  constexpr int ZOFF = YOFF + WY;
-  static_assert(NS % 2 == 0, "even widths only");
-  if constexpr (sizeof(T) == 4) {
-#pragma unroll
-    for (int q = 0; q < NS; q += 2)
-      store16(sp + 2 * q, cv.x * w[0][q], cv.y * w[0][q], cv.x * w[0][q + 1], cv.y * w[0][q + 1]);
-#pragma unroll
-    for (int q = 0; q < WY; q += 4)
-      store16(sp + YOFF + q, q < NS ? w[1][q] : (T)0, q + 1 < NS ? w[1][q + 1] : (T)0,
-              q + 2 < NS ? w[1][q + 2] : (T)0, q + 3 < NS ? w[1][q + 3] : (T)0);
-    if constexpr (DIM == 3) {
-#pragma unroll
-      for (int q = 0; q < WZ; q += 4)
-        store16(sp + ZOFF + q, q < NS ? w[DIM - 1][q] : (T)0, q + 1 < NS ? w[DIM - 1][q + 1] : (T)0,
-                q + 2 < NS ? w[DIM - 1][q + 2] : (T)0, q + 3 < NS ? w[DIM - 1][q + 3] : (T)0);
-    }
-  } else {
-#pragma unroll
-    for (int q = 0; q < NS; ++q) store16(sp + 2 * q, cv.x * w[0][q], cv.y * w[0][q]);
-#pragma unroll
-    for (int q = 0; q < WY; q += 2)
-      store16(sp + YOFF + q, q < NS ? w[1][q] : (T)0, q + 1 < NS ? w[1][q + 1] : (T)0);
-    if constexpr (DIM == 3) {
-#pragma unroll
-      for (int q = 0; q < WZ; q += 2)
-        store16(sp + ZOFF + q, q < NS ? w[DIM - 1][q] : (T)0, q + 1 < NS ? w[DIM - 1][q + 1] : (T)0);
-    }
-  }
-}
+}  // namespace nfx
 
-// Adds one staged point to this lane's accumulators: acc[r] += w_row(r) * (c w_x),
-// w_row the y weight of row grp * rpl + r (2D) or z weight * y weight (3D).
-template <typename T, int DIM, int NS>
-__device__ __forceinline__ void add_slot(const T* sp, int kx, int grp, cplx_t<T> (&acc)[run_rows_per_lane(DIM, NS)]) {
-  using CT = cplx_t<T>;
-  constexpr int RPL = run_rows_per_lane(DIM, NS);
-  constexpr int WY = run_wy(DIM, NS);
-  constexpr int YOFF = round4(2 * NS);
-  constexpr int ZOFF = YOFF + WY;
-  const CT cw = reinterpret_cast<const CT*>(sp)[kx];
-  if constexpr (DIM == 2) {
-    const T* wy = sp + YOFF + grp * RPL;
-#pragma unroll
-    for (int r = 0; r < RPL; ++r) acc[r] = fma_rc(wy[r], cw, acc[r]);
-  } else if constexpr (RPL % NS == 0) {
-    const T* wz = sp + ZOFF + grp * (RPL / NS);
-#pragma unroll
-    for (int zz = 0; zz < RPL / NS; ++zz) {
-      const T z = wz[zz];
-#pragma unroll
-      for (int q = 0; q < NS; ++q) acc[zz * NS + q] = fma_rc(z * sp[YOFF + q], cw, acc[zz * NS + q]);
-    }
-  } else {
-#pragma unroll
-    for (int r = 0; r < RPL; ++r) {
-      const int rho = grp * RPL + r;
-      acc[r] = fma_rc(sp[ZOFF + rho / NS] * sp[YOFF + rho % NS], cw, acc[r]);
-    }
-  }
-}
+#include "nfx_spread_window.cuh"
 
-// Adds one staged point straight to the shared tile at footprint origin `off`.
-// lane_cell: tile offset of this lane's first cell (row grp * rpl, column kx)
-// from the origin, -1 when the lane owns no cell; rows r after the first are
-// r rows further (2D), or r / ns planes and r % ns rows further (3D with rpl a
-// multiple of ns: compile-time in r).
-template <typename T, int DIM, int NS>
-__device__ __forceinline__ void add_slot_direct(const T* sp, int kx, int grp, int off, T* s_re, T* s_im,
-                                                int lane_cell, int row, int plane) {
-  using CT = cplx_t<T>;
-  constexpr int RPL = run_rows_per_lane(DIM, NS);
-  constexpr int NR = run_rows(DIM, NS);
-  constexpr int WY = run_wy(DIM, NS);
-  constexpr int YOFF = round4(2 * NS);
-  constexpr int ZOFF = YOFF + WY;
-  if (lane_cell < 0) return;
-  const CT cw = reinterpret_cast<const CT*>(sp)[kx];
-  T* pr = s_re + off + lane_cell;
-  T* pi = s_im + off + lane_cell;
-  auto add = [&](int o, T w) {
-    atomicAdd(pr + o, w * cw.x);
-    atomicAdd(pi + o, w * cw.y);
-  };
-  if constexpr (DIM == 2) {
-    const T* wy = sp + YOFF + grp * RPL;
-#pragma unroll
-    for (int r = 0; r < RPL; ++r)
-      if (grp * RPL + r < NR) add(r * row, wy[r]);
-  } else if constexpr (RPL % NS == 0) {
-    const T* wz = sp + ZOFF + grp * (RPL / NS);
-    T wy[NS];
-#pragma unroll
-    for (int q = 0; q < NS; ++q) wy[q] = sp[YOFF + q];
-#pragma unroll
-    for (int zz = 0; zz < RPL / NS; ++zz) {
-      const T z = wz[zz];
-#pragma unroll
-      for (int q = 0; q < NS; ++q) add(zz * plane + q * row, z * wy[q]);
-    }
-  } else {
-#pragma unroll
-    for (int r = 0; r < RPL; ++r) {
-      const int rho = grp * RPL + r;
-      if (rho < NR) {
-        const int rz = rho / NS, ry = rho - rz * NS;
-        add((rz - (grp * RPL) / NS) * plane + (ry - (grp * RPL) % NS) * row, sp[ZOFF + rz] * sp[YOFF + ry]);
-      }
-    }
-  }
-}
-
-// 3D batches of 32 points with at least this many run starts (mean run of 4
-// or less) skip the register accumulation and add each point directly: a
-// lane's rpl = 16 rows make a run's walk and flush cost more than the direct
-// adds of a few points.  2D batches always take the walk: a float atomicAdd on
-// shared memory is a compare-and-swap loop (no native float add), so a run's
-// flush of rpl = 2 complex cells per lane costs about as much as adding one
-// point's cells directly, and the walk measured faster than the direct path
-// for batches of mean run 1 to 4 (2D ns = 8: 4M clustered points 167 -> 158
-// us, 0.5M radial points unchanged).
-constexpr int kSparseRuns = 8;
-template <int DIM>
-__device__ __forceinline__ bool direct_batch(unsigned starts) {
-  return DIM == 3 && __popc(starts) >= kSparseRuns;
-}
-
-// Run-merging spread (2D/3D, footprints of at least 32 cells).  Each warp walks
-// a contiguous, cell-ordered slice of the subproblem 32 points at a time: every
-// lane stages one point in a shared slot (stage_slot), then the warp takes the
-// 32 points one after another with lane l accumulating, in registers,
-// footprint column kx = l % ns of rows grp*rpl .. grp*rpl + rpl - 1
-// (grp = l / ns; add_slot).  Consecutive points in the same cell share the
-// footprint, so the registers reach shared memory (atomics, distinct addresses
-// within an instruction) only when the cell changes.  One ballot per batch
-// marks where runs start; the walk goes run by run, each run an unrolled loop
-// with no branch per point.  The next batch's point indices, coordinates and
-// strengths are fetched while the current batch is walked.
-template <typename T, int DIM, int NS, int NW>
-__device__ __forceinline__ void spread_subproblem_runs(const PointArgs<T>& a, const cplx_t<T>* __restrict__ c,
-                                                       cplx_t<T>* __restrict__ fw, int sidx, unsigned char* smem_raw) {
-  using CT = cplx_t<T>;
-  constexpr int G = run_groups(NS);
-  constexpr int RPL = run_rows_per_lane(DIM, NS);
-  constexpr int NR = run_rows(DIM, NS);
-  constexpr int SLOT = run_slot_reals(DIM, NS, (int)sizeof(T));
-  static_assert(SLOT > 0, "run-merging layout does not apply");
-  const Geom& g = a.g;
-  const int tile_cells = g.pad[2] * g.pad[1] * g.pitch;
-  T* s_re = reinterpret_cast<T*>(smem_raw);
-  T* s_im = s_re + tile_cells;
-  // slots start 16-byte aligned after the two tile planes
-  T* s_st = reinterpret_cast<T*>(smem_raw + ((2 * (size_t)tile_cells * sizeof(T) + 15) & ~(size_t)15));
-  const int warp = threadIdx.x >> 5;
-  const int lane = threadIdx.x & 31;
-  const int row = g.pitch;
-  const int plane = g.pitch * g.pad[1];
-  // this lane's column and row group; lanes past the groups mirror the last
-  // group's loads and never flush
-  const int kx = lane % NS;
-  const bool lane_on = lane / NS < G;
-  const int grp = lane_on ? lane / NS : G - 1;
-  T* my_slot = s_st + (warp * 32 + lane) * SLOT;
-  const T* warp_slots = s_st + warp * 32 * SLOT;
-
-  const int b = a.s.sub_bin[sidx];
-  const int k0 = a.s.sub_start[sidx];
-  const int k1 = min(k0 + a.s.maxsub, a.s.bin_start[b + 1]);
-  int o[3];
-  bin_origin(g, b, o[0], o[1], o[2]);
-  for (int t = 0; t < a.n_trans; ++t) {
-    const CT* ct = c + (int64_t)t * a.M;
-    for (int i = threadIdx.x; i < 2 * tile_cells; i += blockDim.x) s_re[i] = (T)0;
-    __syncthreads();
-    const int per = ((k1 - k0 + NW - 1) / NW + 31) / 32 * 32;
-    const int w0 = min(k0 + warp * per, k1);
-    const int w1 = min(w0 + per, k1);
-    // two accumulator sets (alternate points of a run) halve the FMA
-    // dependency chains; flush_run adds them
-    CT acc[RPL], acc2[RPL];
-#pragma unroll
-    for (int r = 0; r < RPL; ++r) acc[r].x = acc[r].y = acc2[r].x = acc2[r].y = (T)0;
-    int run_off = -1;
-    // this lane's first cell (row grp * rpl, column kx) relative to a
-    // footprint's origin; -1 for lanes past the groups
-    const int rho0 = grp * RPL;
-    const int lane_cell = lane_on ? (DIM == 3 ? (rho0 / NS) * plane + (rho0 % NS) * row : rho0 * row) + kx : -1;
-    auto flush_run = [&]() {
-#pragma unroll
-      for (int r = 0; r < RPL; ++r) {
-        acc[r].x += acc2[r].x;
-        acc[r].y += acc2[r].y;
-      }
-      if (lane_cell >= 0) {
-        T* pr = s_re + run_off + lane_cell;
-        T* pi = s_im + run_off + lane_cell;
-#pragma unroll
-        for (int r = 0; r < RPL; ++r) {
-          const int rho = rho0 + r;
-          if (rho < NR) {
-            // offset of row r from this lane's first row
-            int o;
-            if constexpr (DIM == 2) {
-              o = r * row;
-            } else if constexpr (RPL % NS == 0) {
-              o = (r / NS) * plane + (r % NS) * row;
-            } else {
-              o = (rho / NS - rho0 / NS) * plane + (rho % NS - rho0 % NS) * row;
-            }
-            atomicAdd(pr + o, acc[r].x);
-            atomicAdd(pi + o, acc[r].y);
-          }
-        }
-      }
-#pragma unroll
-      for (int r = 0; r < RPL; ++r) acc[r].x = acc[r].y = acc2[r].x = acc2[r].y = (T)0;
-    };
-    // software pipeline: folded coordinates and strength of this lane's point
-    // in the current batch (xn, cn) and the point index of the next batch (pn)
-    T xn[DIM];
-    CT cn;
-    cn.x = cn.y = (T)0;
-#pragma unroll
-    for (int d = 0; d < DIM; ++d) xn[d] = (T)0;
-    int pn = w0 + lane < w1 ? a.s.perm[w0 + lane] : -1;
-    if (pn >= 0) {
-      load_sorted<T, DIM>(a, w0 + lane, xn);
-      cn = ct[pn];
-    }
-    pn = w0 + 32 + lane < w1 ? a.s.perm[w0 + 32 + lane] : -1;
-    for (int kb = w0; kb < w1; kb += 32) {
-      const bool valid = kb + lane < w1;
-      T xv[DIM];
-#pragma unroll
-      for (int d = 0; d < DIM; ++d) xv[d] = xn[d];
-      CT cv = cn;
-      if (pn >= 0) {  // next batch (pn >= 0 exactly when kb + 32 + lane < w1)
-        load_sorted<T, DIM>(a, kb + 32 + lane, xn);
-        cn = ct[pn];
-      }
-      pn = kb + 64 + lane < w1 ? a.s.perm[kb + 64 + lane] : -1;
-      int off = 0;
-      if (valid) {
-        T w[DIM][NS];
-        const bool inside = footprint<T, DIM, NS>(a, xv, o, row, plane, off, w);
-        cv = with_extra(a, kb + lane, cv);
-        if (!inside) {
-          cv.x = cv.y = (T)0;
-          off = 0;
-        }
-        stage_slot<T, DIM, NS>(my_slot, cv, w);
-      }
-      // lane j starts a run when its cell differs from point j-1's
-      int prev = __shfl_up_sync(0xffffffffu, off, 1);
-      if (lane == 0) prev = run_off;
-      const unsigned starts = __ballot_sync(0xffffffffu, valid && off != prev);
-      __syncwarp();
-      const int cnt = min(32, w1 - kb);
-      int j = 0;
-      const T* sp = warp_slots;
-      if (direct_batch<DIM>(starts)) {
-        // short runs: points before the first run start finish the pending
-        // run; every later point is added to shared memory directly
-        const int first = __ffs(starts) - 1;
-        for (; j < first; ++j, sp += SLOT) add_slot<T, DIM, NS>(sp, kx, grp, acc);
-        if (run_off >= 0) flush_run();
-        for (; j < cnt; ++j, sp += SLOT)
-          add_slot_direct<T, DIM, NS>(sp, kx, grp, __shfl_sync(0xffffffffu, off, j), s_re, s_im, lane_cell, row,
-                                      plane);
-        run_off = __shfl_sync(0xffffffffu, off, cnt - 1);  // accumulators are empty
-        j = cnt;
-      }
-      while (j < cnt) {  // one run (or the rest of one) per trip
-        if ((starts >> j) & 1u) {
-          if (run_off >= 0) flush_run();
-          run_off = __shfl_sync(0xffffffffu, off, j);
-        }
-        const unsigned later = j < 31 ? starts >> (j + 1) : 0u;
-        const int je = later != 0u ? min(j + __ffs(later), cnt) : cnt;
-        for (; j + 4 <= je; j += 4, sp += 4 * SLOT) {
-          add_slot<T, DIM, NS>(sp, kx, grp, acc);
-          add_slot<T, DIM, NS>(sp + SLOT, kx, grp, acc2);
-          add_slot<T, DIM, NS>(sp + 2 * SLOT, kx, grp, acc);
-          add_slot<T, DIM, NS>(sp + 3 * SLOT, kx, grp, acc2);
-        }
-        for (; j < je; ++j, sp += SLOT) add_slot<T, DIM, NS>(sp, kx, grp, acc);
-      }
-      __syncwarp();
-    }
-    if (run_off >= 0) flush_run();
-    __syncthreads();
-    flush_tile<T>(g, o, s_re, s_im, fw + (int64_t)t * a.grid_stride);
-    __syncthreads();
-  }
-}
+namespace nfx {
 
 // Spread of one subproblem, footprints below 32 cells (1D, small ns) or with
 // more than 16 rows a lane (3D, ns >= 9).  Points are staged 32 at a time per
@@ -620,21 +327,34 @@ __device__ __forceinline__ void spread_subproblem_cells(const PointArgs<T>& a, c
   }
 }
 
+// Work items of a spread: slices of the sorted points (window spread) or
+// subproblems.
+template <typename T>
+__device__ __forceinline__ int spread_items(const PointArgs<T>& a) {
+  return a.win_part > 0 ? (int)((a.M + a.win_part - 1) / a.win_part) : *a.s.nsub;
+}
 template <typename T, int DIM, int NS, int NW>
-__device__ __forceinline__ void spread_subproblem(const PointArgs<T>& a, const cplx_t<T>* __restrict__ c,
-                                                  cplx_t<T>* __restrict__ fw, int sidx, unsigned char* smem_raw) {
-  if constexpr (run_slot_reals(DIM, NS, (int)sizeof(T)) > 0)
-    spread_subproblem_runs<T, DIM, NS, NW>(a, c, fw, sidx, smem_raw);
-  else
-    spread_subproblem_cells<T, DIM, NS, NW>(a, c, fw, sidx, smem_raw);
+__device__ __forceinline__ void spread_item(const PointArgs<T>& a, const cplx_t<T>* __restrict__ c,
+                                            cplx_t<T>* __restrict__ fw, int item, unsigned char* smem_raw) {
+  if constexpr (WinShape<T, DIM, NS>::on) {
+    spread_window<T, DIM, NS, NW>(a, c, fw, item, smem_raw);
+  } else {
+    spread_subproblem_cells<T, DIM, NS, NW>(a, c, fw, item, smem_raw);
+  }
+}
+
+// CTAs per SM the spread's registers allow for: the window accumulators.
+template <typename T, int DIM, int NS>
+constexpr int spread_min_ctas() {
+  return DIM == 3 || sizeof(T) == 8 ? 2 : (NS <= 8 ? 4 : 3);
 }
 
 template <typename T, int DIM, int NS, int NW>
-__global__ void __launch_bounds__(NW * 32) k_spread(PointArgs<T> a, const cplx_t<T>* __restrict__ c,
+__global__ void __launch_bounds__(NW * 32, spread_min_ctas<T, DIM, NS>()) k_spread(const __grid_constant__ PointArgs<T> a, const cplx_t<T>* __restrict__ c,
                                                     cplx_t<T>* __restrict__ fw) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  const int nsub = *a.s.nsub;
-  for (int sidx = blockIdx.x; sidx < nsub; sidx += gridDim.x) spread_subproblem<T, DIM, NS, NW>(a, c, fw, sidx, smem_raw);
+  const int nitems = spread_items(a);
+  for (int item = blockIdx.x; item < nitems; item += gridDim.x) spread_item<T, DIM, NS, NW>(a, c, fw, item, smem_raw);
 }
 
 // Plane-owner spread (3D, points sparser than cells).  The CTA stages up to
@@ -647,17 +367,6 @@ __global__ void __launch_bounds__(NW * 32) k_spread(PointArgs<T> a, const cplx_t
 // footprint (ns consecutive planes) gives each warp exactly one plane.  Slots
 // are 16-byte aligned (owner_slot_reals): staged with 16-byte stores, read with
 // 8-byte loads of (c w_x re, im), (offset, z) and pairs of y weights.
-template <typename T>
-struct Vec16;
-template <>
-struct Vec16<float> {
-  using type = float4;
-};
-template <>
-struct Vec16<double> {
-  using type = double2;
-};
-
 // The tile of the plane-owner spread holds interleaved complex cells (one
 // 8- or 16-byte load and store per cell update).  Flushed like flush_tile.
 template <typename T>
@@ -1350,8 +1059,7 @@ __global__ void __launch_bounds__(NW * 32) k_spread_batch(const BatchItem<T>* __
   for (int gi = blockIdx.x; gi < total; gi += gridDim.x) {
     const int p = batch_find(sub_prefix, nitems, gi);
     const BatchItem<T>& it = items[p];
-    spread_subproblem<T, DIM, NS, NW>(it.a, (const cplx_t<T>*)it.src, (cplx_t<T>*)it.dst, gi - sub_prefix[p],
-                                      smem_raw);
+    spread_item<T, DIM, NS, NW>(it.a, (const cplx_t<T>*)it.src, (cplx_t<T>*)it.dst, gi - sub_prefix[p], smem_raw);
     __syncthreads();
   }
 }
@@ -1544,7 +1252,27 @@ __global__ void __launch_bounds__(NW * 32) k_grad(PointArgs<T> a, const cplx_t<T
 template <typename T, int DIM, int NS>
 struct Launch {
   static constexpr int NW = warps_per_cta(sizeof(T), DIM, NS);
+  static constexpr int SW = win_warps<T, DIM, NS>();  // of the spread
   static size_t tile_smem(const Geom& g) { return (size_t)g.pad[2] * g.pad[1] * g.pitch * sizeof(cplx_t<T>); }
+
+  // Chooses the work items of a spread of M_total points (over all problems of
+  // the launch, which has room for `ctas` CTAs at a time); returns a bound on
+  // this problem's items.
+  static int64_t split_items(int64_t M_total, int ctas, PointArgs<T>& a) {
+    if constexpr (WinShape<T, DIM, NS>::on) {
+      a.win_part = win_part_points(DIM, M_total, ctas);
+      return (a.M + a.win_part - 1) / a.win_part;
+    } else {
+      return a.s.max_subs;
+    }
+  }
+  // Shared memory of the spread kernels (plain and batched) on a grid geometry.
+  static size_t smem_spread(const Geom& g) {
+    if constexpr (WinShape<T, DIM, NS>::on)
+      return win_smem_bytes<T, DIM, NS>();
+    else
+      return spread_smem_bytes(sizeof(T), DIM, NS, g);
+  }
 
   template <typename K>
   static cudaError_t prep(K kernel, size_t smem, int& grid, int64_t max_subs) {
@@ -1554,12 +1282,16 @@ struct Launch {
   static cudaError_t spread(const PointArgs<T>& a, const cplx_t<T>* c, cplx_t<T>* fw, cudaStream_t st) {
     int grid = 0;
     if constexpr (DIM == 3 && NS >= 4) {
-      // threads per point (Geom::spread_mode): the whole CTA (warps own tile
-      // planes; by default when points are sparser than grid cells: runs of
-      // same-cell points are rare, and the plane-owner spread needs no
-      // shared-memory atomics) or one warp (lanes own footprint columns)
+      // The plane-owner spread where no register window exists (widths from 10)
+      // and points are sparser than grid cells, and for complex128 of width 8 on
+      // such sets: its 9^3-cell windows hold about one point there, and their
+      // reds cost more than the tile (100 k points on 96^3: window 355 us, owner
+      // 265; 300 k: 592 against 556; widths 4 and 6: 83 against 103, 181 against
+      // 265).  complex64 windows win at every density (1e4 points on 128^3: 52
+      // against 99 us, 8M on 256^3: 1725 against 3645).
       const bool sparse = a.M < (int64_t)a.g.nf[0] * a.g.nf[1] * a.g.nf[2];
-      if (a.g.spread_mode == NFX_PER_POINT_CTA || (a.g.spread_mode == NFX_PER_POINT_AUTO && sparse)) {
+      const bool window = WinShape<T, DIM, NS>::on && (sizeof(T) == 4 || NS <= 6 || !sparse);
+      if (a.g.spread_mode == NFX_PER_POINT_CTA || (a.g.spread_mode == NFX_PER_POINT_AUTO && sparse && !window)) {
         // the tile's row pitch is this kernel's own (footprint offsets follow it)
         PointArgs<T> ao = a;
         ao.g.pitch = owner_pitch(a.g.pitch, a.g.pad[0], NS, (int)sizeof(T));
@@ -1570,10 +1302,12 @@ struct Launch {
         return cudaGetLastError();
       }
     }
-    size_t smem = spread_smem_bytes(sizeof(T), DIM, NS, a.g);
-    cudaError_t e = prep(k_spread<T, DIM, NS, NW>, smem, grid, a.s.max_subs);
+    const size_t smem = smem_spread(a.g);
+    PointArgs<T> as = a;
+    cudaError_t e = kernel_grid(reinterpret_cast<const void*>(k_spread<T, DIM, NS, SW>), SW * 32, smem, INT32_MAX, grid);
     if (e != cudaSuccess) return e;
-    k_spread<T, DIM, NS, NW><<<grid, NW * 32, smem, st>>>(a, c, fw);
+    grid = (int)std::max<int64_t>(1, std::min<int64_t>(grid, split_items(as.M, grid, as)));
+    k_spread<T, DIM, NS, SW><<<grid, SW * 32, smem, st>>>(as, c, fw);
     return cudaGetLastError();
   }
   template <int MODE>
@@ -1629,13 +1363,14 @@ struct Launch {
 template <typename T, int DIM, int NS>
 struct BatchLaunch {
   static constexpr int NW = warps_per_cta(sizeof(T), DIM, NS);
+  static constexpr int SW = win_warps<T, DIM, NS>();
   static cudaError_t spread(const void* items, int n, const int* prefix, int64_t max_subs, size_t smem,
                             cudaStream_t st) {
     int grid = 0;
-    cudaError_t e = kernel_grid(reinterpret_cast<const void*>(k_spread_batch<T, DIM, NS, NW>), NW * 32, smem, max_subs,
+    cudaError_t e = kernel_grid(reinterpret_cast<const void*>(k_spread_batch<T, DIM, NS, SW>), SW * 32, smem, max_subs,
                                 grid);
     if (e != cudaSuccess) return e;
-    k_spread_batch<T, DIM, NS, NW><<<grid, NW * 32, smem, st>>>((const BatchItem<T>*)items, n, prefix);
+    k_spread_batch<T, DIM, NS, SW><<<grid, SW * 32, smem, st>>>((const BatchItem<T>*)items, n, prefix);
     return cudaGetLastError();
   }
   static cudaError_t interp(const void* items, int n, const int* prefix, int64_t max_subs, size_t smem,
@@ -1661,6 +1396,36 @@ cudaError_t dispatch_batch(int ns, bool spread, const void* items, int n, const 
 #undef NFX_CASE
     default:
       return cudaErrorInvalidValue;
+  }
+}
+
+// Shared memory of the spread of one problem (the batched launches take the
+// largest of theirs).
+template <typename T, int DIM>
+size_t spread_smem_dim(int ns, const Geom& g) {
+  switch (ns) {
+#define NFX_CASE(N) \
+  case N:           \
+    return Launch<T, DIM, N>::smem_spread(g);
+    NFX_CASE(2) NFX_CASE(4) NFX_CASE(6) NFX_CASE(8) NFX_CASE(10) NFX_CASE(12) NFX_CASE(14) NFX_CASE(16)
+#undef NFX_CASE
+    default:
+      return 0;
+  }
+}
+
+// Work items of one problem of a batched spread (Launch::split_items).
+template <typename T, int DIM>
+int64_t split_spread_items(int ns, int64_t M_total, PointArgs<T>& a) {
+  const int ctas = num_sms() * (DIM == 2 ? 4 : 2);
+  switch (ns) {
+#define NFX_CASE(N) \
+  case N:           \
+    return Launch<T, DIM, N>::split_items(M_total, ctas, a);
+    NFX_CASE(2) NFX_CASE(4) NFX_CASE(6) NFX_CASE(8) NFX_CASE(10) NFX_CASE(12) NFX_CASE(14) NFX_CASE(16)
+#undef NFX_CASE
+    default:
+      return 0;
   }
 }
 
@@ -1714,6 +1479,7 @@ PointArgs<T> make_args(const Geom& g, double beta, double kc, int64_t M, int n_t
   a.M = M;
   a.n_trans = n_trans;
   a.grid_stride = (int64_t)g.nf[0] * g.nf[1] * g.nf[2];
+  a.win_part = 0;
   a.tma = 0;
   a.status = nullptr;
   a.g = g;
