@@ -23,6 +23,7 @@ struct SortLayout {
   int bits;         // bits of the composite key
   int npass;        // radix passes (digits of dbits bits, least significant first)
   int dbits;
+  int chunk;        // elements of one chunk (one CTA) of a radix pass
   int nchunks;      // chunks of one radix pass
   int maxsub;       // points per subproblem
   int64_t max_subs; // upper bound on the number of subproblems
@@ -73,7 +74,10 @@ struct SortView {
 };
 
 void radix_plan(int nbins, int ncell, int& cbits, int& bits, int& npass, int& dbits);
-int radix_chunk();
+// Elements per chunk of a sort of M points, and the rows of its count matrix
+// (at least one per chunk).
+int radix_chunk(int64_t M);
+int radix_count_rows(int64_t M);
 // out[i] = bin of point i (composite key / cells per tile)
 cudaError_t bin_keys_of(const SortLayout& L, const int* K, int* out, cudaStream_t st);
 

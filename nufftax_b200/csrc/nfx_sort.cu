@@ -8,7 +8,7 @@
 // tile edge, x-fastest) and cell that cell's index inside the tile (cbits =
 // bits of cells per tile); the permutation is the STABLE sort by (bin, cell),
 // equal to numpy.argsort(bin * cells_per_tile + cell, kind="stable") bit for
-// bit.  Work is split into chunks of 4096 consecutive elements, one CTA each:
+// bit.  Work is split into chunks of consecutive elements (radix_chunk), one CTA each:
 //
 // (1) k_sort_keys computes K for every point (one pass over the coordinates)
 //     and each chunk's histogram of the first radix digit, written as row
@@ -79,19 +79,27 @@ __device__ __forceinline__ void cell_keys(const T (&c)[DIM], const Geom& g, int 
 }
 
 constexpr int kRadixThreads = 256;
+// Elements per thread of a chunk (one CTA).  Up to 303 k points 4: 4096-element
+// chunks would leave half of the SMs idle, and a chunk's latency (its ranking
+// rounds) is what a small sort waits for.  Above, 16: a chunk clears and scans
+// 8 x 2^bits counters whatever its length.  Both scatter passes, 16 -> 4: 1 k
+// points (8 bits) 15.7 -> 8.9 us, 200 k (7 bits) 17.6 -> 10.2, 300 k (9 bits) 21.8
+// -> 15.9, but 524 k (10 bits) 25.6 -> 35.6; the column scans take 4.5 -> 6.8 at
+// 300 k, the keys 8.0 -> 3.7.
 constexpr int kRadixItems = 16;
-constexpr int kRadixChunk = kRadixThreads * kRadixItems;  // elements per chunk (one CTA)
+constexpr int kRadixItemsSmall = 4;
+constexpr int64_t kRadixSmallM = 148 * 2 * kRadixThreads * kRadixItemsSmall;  // two CTAs an SM
 
 // ---- (1) composite keys + the first digit's per-chunk counts ---------------
-// One CTA per chunk of kRadixChunk consecutive points: K = bin << cbits | cell
+// One CTA per chunk of consecutive points: K = bin << cbits | cell
 // for every point, and the chunk's histogram of digit 0 as row `chunk` of
 // counts (chunk-major, so the row is one coalesced write).
 // T3: the points are type-3 sources or targets (Geom::t3_mode), a separate
 // instantiation so the common kernel carries no type-3 code.
 // f[d] (nullptr: not wanted): every point's folded coordinates in input order,
 // the payload the scatter passes then carry into sorted order.
-template <typename T, int DIM, bool T3>
-__global__ void __launch_bounds__(kRadixThreads) k_sort_keys(const T* __restrict__ x, const T* __restrict__ y,
+template <typename T, int DIM, bool T3, int ITEMS>
+__global__ void __launch_bounds__(kRadixThreads, ITEMS > 4 ? 4 : 1) k_sort_keys(const T* __restrict__ x, const T* __restrict__ y,
                                                             const T* __restrict__ z, int M, Geom g, int ns_half,
                                                             int cbits, int dbits, int* __restrict__ K,
                                                             int* __restrict__ counts, T* __restrict__ f0,
@@ -101,18 +109,18 @@ __global__ void __launch_bounds__(kRadixThreads) k_sort_keys(const T* __restrict
   const int mask = B - 1;
   for (int i = threadIdx.x; i < B; i += blockDim.x) s_h[i] = 0;
   __syncthreads();
-  const int c0 = blockIdx.x * kRadixChunk;
+  const int c0 = blockIdx.x * (kRadixThreads * ITEMS);
   const T* cs[3] = {x, y, z};
   // all coordinate loads first, so they are in flight together
-  T cv[kRadixItems][DIM];
+  T cv[ITEMS][DIM];
 #pragma unroll
-  for (int u = 0; u < kRadixItems; ++u) {
+  for (int u = 0; u < ITEMS; ++u) {
     const int p = c0 + u * kRadixThreads + threadIdx.x;
 #pragma unroll
     for (int d = 0; d < DIM; ++d) cv[u][d] = p < M ? cs[d][p] : (T)0;
   }
 #pragma unroll
-  for (int u = 0; u < kRadixItems; ++u) {
+  for (int u = 0; u < ITEMS; ++u) {
     const int p = c0 + u * kRadixThreads + threadIdx.x;
     if (p < M) {
       int kb, kc;
@@ -134,6 +142,7 @@ __global__ void __launch_bounds__(kRadixThreads) k_sort_keys(const T* __restrict
 }
 
 // Per-chunk counts of digit (K >> shift) & (B - 1), for the passes after the first.
+template <int ITEMS>
 __global__ void __launch_bounds__(kRadixThreads) k_digit_count(const int* __restrict__ kin, int M, int shift,
                                                               int dbits, int* __restrict__ counts) {
   extern __shared__ int s_h[];
@@ -141,15 +150,15 @@ __global__ void __launch_bounds__(kRadixThreads) k_digit_count(const int* __rest
   const int mask = B - 1;
   for (int i = threadIdx.x; i < B; i += blockDim.x) s_h[i] = 0;
   __syncthreads();
-  const int c0 = blockIdx.x * kRadixChunk;
-  int key[kRadixItems];
+  const int c0 = blockIdx.x * (kRadixThreads * ITEMS);
+  int key[ITEMS];
 #pragma unroll
-  for (int u = 0; u < kRadixItems; ++u) {
+  for (int u = 0; u < ITEMS; ++u) {
     const int p = c0 + u * kRadixThreads + threadIdx.x;
     key[u] = p < M ? kin[p] : -1;
   }
 #pragma unroll
-  for (int u = 0; u < kRadixItems; ++u)
+  for (int u = 0; u < ITEMS; ++u)
     if (key[u] >= 0) atomicAdd(&s_h[(key[u] >> shift) & mask], 1);
   __syncthreads();
   int* row = counts + (size_t)blockIdx.x * B;
@@ -221,11 +230,11 @@ __global__ void __launch_bounds__(kScanDigits * kScanGroups) k_col_scan(int* __r
 // chunk's digit starts and each digit's output offset.
 // Shared-memory ints of the region that first holds the per-warp digit counts
 // and then the staged chunk (keys, values and PD payload words per element).
-__host__ __device__ constexpr int radix_region_ints(int B, int PD) {
-  return (kRadixThreads / 32) * B > (2 + PD) * kRadixChunk ? (kRadixThreads / 32) * B : (2 + PD) * kRadixChunk;
+__host__ __device__ constexpr int radix_region_ints(int B, int PD, int chunk) {
+  return (kRadixThreads / 32) * B > (2 + PD) * chunk ? (kRadixThreads / 32) * B : (2 + PD) * chunk;
 }
-__host__ __device__ constexpr size_t radix_smem_bytes(int B, int PD) {
-  return (size_t)(radix_region_ints(B, PD) + 2 * B) * sizeof(int);
+__host__ __device__ constexpr size_t radix_smem_bytes(int B, int PD, int chunk) {
+  return (size_t)(radix_region_ints(B, PD, chunk) + 2 * B) * sizeof(int);
 }
 
 // Float words carried with every element through a pass (the folded
@@ -244,7 +253,7 @@ struct RadixPayload {
 // pass whose digit is the bin): CTA 0 writes the bin starts (the exclusive
 // scan of the digit totals), bstart[0..nbins].  DB = dbits (compile time, so
 // the ranking's ballots unroll); DPT = digits per thread, max(1, 2^DB / 256).
-template <int DB, int PD, int DPT = (((1 << DB) + kRadixThreads - 1) / kRadixThreads)>
+template <int DB, int PD, int ITEMS, int DPT = (((1 << DB) + kRadixThreads - 1) / kRadixThreads)>
 __global__ void __launch_bounds__(kRadixThreads, 3) k_radix_scatter(const int* __restrict__ kin,
                                                                 const int* __restrict__ vin, int M, int shift,
                                                                 int dbits, const int* __restrict__ prefix,
@@ -254,25 +263,26 @@ __global__ void __launch_bounds__(kRadixThreads, 3) k_radix_scatter(const int* _
                                                                 int nbins) {
   extern __shared__ int smem[];
   __shared__ int s_warp[32];
+  constexpr int kChunk = kRadixThreads * ITEMS;
   constexpr int W = kRadixThreads / 32;
   constexpr int B = 1 << DB;
   constexpr int mask = B - 1;
   int* s_hw = smem;                                 // [W][B] per-warp digit counts
-  int* s_key = smem;                                // [kRadixChunk] staged keys (after ranking)
-  int* s_val = smem + kRadixChunk;                  // [kRadixChunk] staged values
-  float* s_pay = reinterpret_cast<float*>(smem + 2 * kRadixChunk);  // [PD][kRadixChunk] staged payload
-  int* s_dstart = smem + radix_region_ints(B, PD);  // [B] digit starts within the chunk
+  int* s_key = smem;                                // [kChunk] staged keys (after ranking)
+  int* s_val = smem + kChunk;                  // [kChunk] staged values
+  float* s_pay = reinterpret_cast<float*>(smem + 2 * kChunk);  // [PD][kChunk] staged payload
+  int* s_dstart = smem + radix_region_ints(B, PD, kChunk);  // [B] digit starts within the chunk
   int* s_gofs = s_dstart + B;                       // [B] output index - staged index, per digit
   for (int i = threadIdx.x; i < W * B; i += blockDim.x) s_hw[i] = 0;
   const int ch = blockIdx.x;
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int c0 = ch * kRadixChunk;
-  const int wbase = c0 + w * (kRadixItems * 32);
+  const int c0 = ch * kChunk;
+  const int wbase = c0 + w * (ITEMS * 32);
   // keys now; values (and payload) only when the chunk is staged, so that the
   // unrolled ranking does not hold them in registers
-  int key[kRadixItems], rk[kRadixItems];
+  int key[ITEMS], rk[ITEMS];
 #pragma unroll
-  for (int r = 0; r < kRadixItems; ++r) {
+  for (int r = 0; r < ITEMS; ++r) {
     const int p = wbase + r * 32 + lane;
     key[r] = p < M ? kin[p] : -1;
   }
@@ -297,7 +307,7 @@ __global__ void __launch_bounds__(kRadixThreads, 3) k_radix_scatter(const int* _
   const unsigned lt = (1u << lane) - 1u;
   int* hw = s_hw + w * B;
 #pragma unroll
-  for (int r = 0; r < kRadixItems; ++r) {
+  for (int r = 0; r < ITEMS; ++r) {
     const int d = key[r] >= 0 ? (key[r] >> shift) & mask : -1;
     // DB + 1 bits: digits shifted by one so the invalid lanes (-1) stay apart
     const unsigned peers = peer_mask<DB + 1>(d);
@@ -346,7 +356,7 @@ __global__ void __launch_bounds__(kRadixThreads, 3) k_radix_scatter(const int* _
   __syncthreads();
   // staged (digit-ordered) index of every element
 #pragma unroll
-  for (int r = 0; r < kRadixItems; ++r) {
+  for (int r = 0; r < ITEMS; ++r) {
     if (key[r] >= 0) {
       const int d = (key[r] >> shift) & mask;
       rk[r] += s_dstart[d] + hw[d];
@@ -354,14 +364,14 @@ __global__ void __launch_bounds__(kRadixThreads, 3) k_radix_scatter(const int* _
   }
   __syncthreads();  // the per-warp counts are dead: the region now holds the staged chunk
   {
-    int val[kRadixItems];
+    int val[ITEMS];
 #pragma unroll
-    for (int r = 0; r < kRadixItems; ++r) {
+    for (int r = 0; r < ITEMS; ++r) {
       const int p = wbase + r * 32 + lane;
       val[r] = key[r] >= 0 ? (vin != nullptr ? vin[p] : p) : 0;
     }
 #pragma unroll
-    for (int r = 0; r < kRadixItems; ++r) {
+    for (int r = 0; r < ITEMS; ++r) {
       if (key[r] >= 0) {
         s_key[rk[r]] = key[r];
         s_val[rk[r]] = val[r];
@@ -370,18 +380,18 @@ __global__ void __launch_bounds__(kRadixThreads, 3) k_radix_scatter(const int* _
   }
 #pragma unroll
   for (int d = 0; d < PD; ++d) {
-    float pv[kRadixItems];
+    float pv[ITEMS];
 #pragma unroll
-    for (int r = 0; r < kRadixItems; ++r) {
+    for (int r = 0; r < ITEMS; ++r) {
       const int p = wbase + r * 32 + lane;
       pv[r] = p < M ? pay.in[d][p] : 0.f;
     }
 #pragma unroll
-    for (int r = 0; r < kRadixItems; ++r)
-      if (key[r] >= 0) s_pay[d * kRadixChunk + rk[r]] = pv[r];
+    for (int r = 0; r < ITEMS; ++r)
+      if (key[r] >= 0) s_pay[d * kChunk + rk[r]] = pv[r];
   }
   __syncthreads();
-  const int n_here = M - c0 < kRadixChunk ? M - c0 : kRadixChunk;
+  const int n_here = M - c0 < kChunk ? M - c0 : kChunk;
   for (int i = threadIdx.x; i < n_here; i += blockDim.x) {
     const int k = s_key[i];
     const int gpos = s_gofs[(k >> shift) & mask] + i;
@@ -389,7 +399,7 @@ __global__ void __launch_bounds__(kRadixThreads, 3) k_radix_scatter(const int* _
       kout[gpos] = k;
       vout[gpos] = s_val[i];
 #pragma unroll
-      for (int d = 0; d < PD; ++d) pay.out[d][gpos] = s_pay[d * kRadixChunk + i];
+      for (int d = 0; d < PD; ++d) pay.out[d][gpos] = s_pay[d * kChunk + i];
     }
   }
 }
@@ -397,26 +407,27 @@ __global__ void __launch_bounds__(kRadixThreads, 3) k_radix_scatter(const int* _
 // The scatter instantiation for dbits-bit digits (1..11) and PD payload arrays.
 using ScatterFn = void (*)(const int*, const int*, int, int, int, const int*, const int*, int*, int*, RadixPayload,
                            int*, int);
-template <int PD>
+template <int PD, int ITEMS>
 static ScatterFn scatter_for_digits(int dbits) {
   switch (dbits) {
-    case 1: return k_radix_scatter<1, PD>;
-    case 2: return k_radix_scatter<2, PD>;
-    case 3: return k_radix_scatter<3, PD>;
-    case 4: return k_radix_scatter<4, PD>;
-    case 5: return k_radix_scatter<5, PD>;
-    case 6: return k_radix_scatter<6, PD>;
-    case 7: return k_radix_scatter<7, PD>;
-    case 8: return k_radix_scatter<8, PD>;
-    case 9: return k_radix_scatter<9, PD>;
-    case 10: return k_radix_scatter<10, PD>;
-    default: return k_radix_scatter<11, PD>;
+    case 1: return k_radix_scatter<1, PD, ITEMS>;
+    case 2: return k_radix_scatter<2, PD, ITEMS>;
+    case 3: return k_radix_scatter<3, PD, ITEMS>;
+    case 4: return k_radix_scatter<4, PD, ITEMS>;
+    case 5: return k_radix_scatter<5, PD, ITEMS>;
+    case 6: return k_radix_scatter<6, PD, ITEMS>;
+    case 7: return k_radix_scatter<7, PD, ITEMS>;
+    case 8: return k_radix_scatter<8, PD, ITEMS>;
+    case 9: return k_radix_scatter<9, PD, ITEMS>;
+    case 10: return k_radix_scatter<10, PD, ITEMS>;
+    default: return k_radix_scatter<11, PD, ITEMS>;
   }
 }
+template <int ITEMS>
 static ScatterFn scatter_for(int dbits, int PD) {
-  return PD == 0 ? scatter_for_digits<0>(dbits)
-                 : (PD == 1 ? scatter_for_digits<1>(dbits)
-                            : (PD == 2 ? scatter_for_digits<2>(dbits) : scatter_for_digits<3>(dbits)));
+  return PD == 0 ? scatter_for_digits<0, ITEMS>(dbits)
+                 : (PD == 1 ? scatter_for_digits<1, ITEMS>(dbits)
+                            : (PD == 2 ? scatter_for_digits<2, ITEMS>(dbits) : scatter_for_digits<3, ITEMS>(dbits)));
 }
 
 // ---- (3) bin starts and subproblems ----------------------------------------
@@ -515,18 +526,33 @@ __global__ void k_subproblems(const int* __restrict__ bin_start, int nbins, int 
 // [-ns/2, ns/2] (nufft3.py:176-213, 390-394), in double before one rounding.
 constexpr int kMaxQuad = 32;
 
+// s_qw[m], m < nh: the trapezoid's weights phi(z) w of the nodes z >= 0 in
+// ascending order, doubled for z > 0 (phi and the cosine are even): z = (m + 1/2)
+// dz for an even node count, m dz for an odd one.  The cosines of the equally
+// spaced nodes come from one sincos by rotation (at most 16 steps, each an error
+// of about one rounding).
 template <typename T>
 __device__ __forceinline__ cplx_t<T> t3_factor(const T (&xr)[3], int dim, const Geom& g, int nq, double dz,
                                                const double* __restrict__ s_qw) {
   const T3Params* p = g.t3;
+  const int nh = (nq + 1) / 2;
   double phase = 0.0, phi_prod = 1.0;
   for (int d = 0; d < dim; ++d) {
     if (g.t3_mode == 1) {
       phase += p->D[d] * (double)xr[d];
     } else {
       const double sr = (double)t3_rescaled(xr[d], d, g);
+      double s0, c0;
+      sincos(0.5 * sr * dz, &s0, &c0);
+      const double cd = c0 * c0 - s0 * s0, sd = 2.0 * s0 * c0;  // one node spacing
+      double cq = nq % 2 == 0 ? c0 : 1.0, sq = nq % 2 == 0 ? s0 : 0.0;
       double acc = 0.0;
-      for (int q = 0; q < nq; ++q) acc += s_qw[q] * cos(sr * (-0.5 * dz * (nq - 1) + q * dz));
+      for (int m = 0; m < nh; ++m) {
+        acc += s_qw[m] * cq;
+        const double cn = cq * cd - sq * sd;
+        sq = sq * cd + cq * sd;
+        cq = cn;
+      }
       phi_prod *= acc;
       phase += ((double)xr[d] - p->D[d]) * p->C[d];
     }
@@ -554,18 +580,20 @@ __global__ void __launch_bounds__(256) k_sorted_coords(const T* __restrict__ x, 
                                                        const T* __restrict__ z, const int* __restrict__ perm, int M,
                                                        Geom g, int nspread, T* __restrict__ o0, T* __restrict__ o1,
                                                        T* __restrict__ o2, cplx_t<T>* __restrict__ extra) {
-  constexpr int Q = kCoordItems;
-  // trapezoid nodes and weights phi(z_q) w_q of the type-3 targets' phihat
+  // type-3 points: one per thread (their factor is double arithmetic, not memory)
+  constexpr int Q = T3 ? 1 : kCoordItems;
+  // weights phi(z_q) w_q of the type-3 targets' phihat (t3_factor)
   __shared__ double s_qw[kMaxQuad];
   const double j2 = nspread / 2.0;
   const int nq = min(max((int)(4 + 3.0 * j2), 20), kMaxQuad);
   const double dz = 2.0 * j2 / (nq - 1);
   if (T3 && g.t3_mode == 2) {
-    for (int q = threadIdx.x; q < nq; q += blockDim.x) {
+    for (int m = threadIdx.x; m < (nq + 1) / 2; m += blockDim.x) {
+      const int q = nq / 2 + m;  // node of the reference's order, -j2 + q dz >= 0
       const double zq = -j2 + q * dz;
       const double arg = 1.0 - g.t3_kc * zq * zq;
       const double phi = arg >= 0.0 ? exp(g.t3_beta * (sqrt(arg > 0.0 ? arg : 0.0) - 1.0)) : 0.0;
-      s_qw[q] = phi * ((q == 0 || q == nq - 1) ? dz / 2 : dz);
+      s_qw[m] = phi * (q == nq - 1 ? dz / 2 : dz) * (nq % 2 == 1 && m == 0 ? 1.0 : 2.0);
     }
     __syncthreads();
   }
@@ -573,7 +601,7 @@ __global__ void __launch_bounds__(256) k_sorted_coords(const T* __restrict__ x, 
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < ngroups; t += gridDim.x * blockDim.x) {
     const int i0 = Q * t;
     int p[Q];
-    if (i0 + Q - 1 < M) {
+    if (Q % 4 == 0 && i0 + Q - 1 < M) {
 #pragma unroll
       for (int h = 0; h < Q / 4; ++h) {
         const int4 v = *reinterpret_cast<const int4*>(perm + i0 + 4 * h);  // 16-byte aligned
@@ -600,7 +628,7 @@ __global__ void __launch_bounds__(256) k_sorted_coords(const T* __restrict__ x, 
       T r[Q];
 #pragma unroll
       for (int j = 0; j < Q; ++j) r[j] = T3 ? point_fold(v[d][j], d, g) : scaled_coord(v[d][j], g.nf[d], g.prenorm);
-      if (i0 + Q - 1 < M) {
+      if (Q % 4 == 0 && i0 + Q - 1 < M) {
 #pragma unroll
         for (int h = 0; h < Q / 4; ++h) {
           const T rq[4] = {r[4 * h], r[4 * h + 1], r[4 * h + 2], r[4 * h + 3]};
@@ -643,7 +671,16 @@ void radix_plan(int nbins, int ncell, int& cbits, int& bits, int& npass, int& db
   dbits = (bits + npass - 1) / npass;
 }
 
-int radix_chunk() { return kRadixChunk; }
+int radix_chunk(int64_t M) { return kRadixThreads * (M <= kRadixSmallM ? kRadixItemsSmall : kRadixItems); }
+
+// Just above kRadixSmallM the longer chunks need fewer rows than just below; the
+// reserve then shrinks more slowly than the per-point arrays grow, so that a
+// workspace that fits M points fits every smaller M.
+int radix_count_rows(int64_t M) {
+  const int64_t rows = (M + radix_chunk(M) - 1) / radix_chunk(M);
+  const int64_t reserve = kRadixSmallM / (kRadixThreads * kRadixItemsSmall) - (M - kRadixSmallM) / 4096;
+  return (int)(M > kRadixSmallM && reserve > rows ? reserve : rows);
+}
 
 cudaError_t bin_keys_of(const SortLayout& L, const int* K, int* out, cudaStream_t st) {
   if (L.M == 0) return cudaSuccess;
@@ -652,10 +689,11 @@ cudaError_t bin_keys_of(const SortLayout& L, const int* K, int* out, cudaStream_
   return cudaGetLastError();
 }
 
-template <typename T>
-cudaError_t launch_sort(const SortLayout& L, const Geom& g, int ns, const void* x, const void* y, const void* z,
+template <typename T, int ITEMS>
+static cudaError_t launch_sort_items(const SortLayout& L, const Geom& g, int ns, const void* x, const void* y, const void* z,
                         int64_t M, const SortPtrs& P, cudaStream_t st) {
   const int B = 1 << L.dbits;
+  constexpr int kChunk = kRadixThreads * ITEMS;
   cudaError_t e = cudaSuccess;
   // float coordinates of non-type-3 points ride through the passes as payload
   // (the layout then holds coord_tmp); otherwise k_sorted_coords gathers them
@@ -664,15 +702,15 @@ cudaError_t launch_sort(const SortLayout& L, const Geom& g, int ns, const void* 
   if (M > 0) {
     const size_t hist_smem = (size_t)B * sizeof(int);
     // digits per thread of the scatter: 2^dbits / 256, at least 1
-    const ScatterFn scatter = scatter_for(L.dbits, PD);
-    e = ensure_smem(reinterpret_cast<const void*>(scatter), radix_smem_bytes(B, PD));
+    const ScatterFn scatter = scatter_for<ITEMS>(L.dbits, PD);
+    e = ensure_smem(reinterpret_cast<const void*>(scatter), radix_smem_bytes(B, PD, kChunk));
     if (e == cudaSuccess) e = prefer_max_smem(reinterpret_cast<const void*>(scatter));
     if (e != cudaSuccess) return e;
     const unsigned scan_grid = (unsigned)((B + kScanDigits - 1) / kScanDigits);
     auto keys = g.t3_mode != 0
-                    ? (g.dim == 1 ? k_sort_keys<T, 1, true> : (g.dim == 2 ? k_sort_keys<T, 2, true> : k_sort_keys<T, 3, true>))
-                    : (g.dim == 1 ? k_sort_keys<T, 1, false>
-                                  : (g.dim == 2 ? k_sort_keys<T, 2, false> : k_sort_keys<T, 3, false>));
+                    ? (g.dim == 1 ? k_sort_keys<T, 1, true, ITEMS> : (g.dim == 2 ? k_sort_keys<T, 2, true, ITEMS> : k_sort_keys<T, 3, true, ITEMS>))
+                    : (g.dim == 1 ? k_sort_keys<T, 1, false, ITEMS>
+                                  : (g.dim == 2 ? k_sort_keys<T, 2, false, ITEMS> : k_sort_keys<T, 3, false, ITEMS>));
     // ping-pong so that the last pass writes (keys_sorted, perm[, coord]); the
     // keys kernel writes the input-order coordinates into the buffer the first
     // pass does not write
@@ -685,7 +723,7 @@ cudaError_t launch_sort(const SortLayout& L, const Geom& g, int ns, const void* 
     void* const* cin = cfirst;
     for (int ps = 0; ps < L.npass; ++ps) {
       const int shift = ps * L.dbits;
-      if (ps > 0) k_digit_count<<<L.nchunks, kRadixThreads, hist_smem, st>>>(kin, (int)M, shift, L.dbits, P.counts);
+      if (ps > 0) k_digit_count<ITEMS><<<L.nchunks, kRadixThreads, hist_smem, st>>>(kin, (int)M, shift, L.dbits, P.counts);
       k_col_scan<<<scan_grid, kScanDigits * kScanGroups, 0, st>>>(P.counts, L.nchunks, B, P.totals);
       const bool to_final = ((L.npass - 1 - ps) % 2) == 0;
       int* kout = to_final ? P.keys_sorted : P.keys_tmp;
@@ -698,7 +736,7 @@ cudaError_t launch_sort(const SortLayout& L, const Geom& g, int ns, const void* 
       }
       // the last pass's digit is the bin when it starts at the cell bits
       int* bstart = (ps == L.npass - 1 && shift == L.cbits) ? P.bin_start : nullptr;
-      scatter<<<L.nchunks, kRadixThreads, radix_smem_bytes(B, PD), st>>>(
+      scatter<<<L.nchunks, kRadixThreads, radix_smem_bytes(B, PD, kChunk), st>>>(
           kin, vin, (int)M, shift, L.dbits, P.counts, P.totals, kout, vout, pay, bstart, g.nbins);
       kin = kout;
       vin = vout;
@@ -713,8 +751,8 @@ cudaError_t launch_sort(const SortLayout& L, const Geom& g, int ns, const void* 
                                            : (g.dim == 2 ? k_sorted_coords<T, 2, true> : k_sorted_coords<T, 3, true>))
                              : (g.dim == 1 ? k_sorted_coords<T, 1, false>
                                            : (g.dim == 2 ? k_sorted_coords<T, 2, false> : k_sorted_coords<T, 3, false>));
-    const int cgrid =
-        (int)std::max<int64_t>(1, std::min<int64_t>((M / kCoordItems + 256) / 256, (int64_t)num_sms() * 8));
+    const int items = g.t3_mode != 0 ? 1 : kCoordItems;
+    const int cgrid = (int)std::max<int64_t>(1, std::min<int64_t>((M / items + 256) / 256, (int64_t)num_sms() * 8));
     sc<<<cgrid, 256, 0, st>>>((const T*)x, (const T*)y, (const T*)z, P.perm, (int)M, g, ns, (T*)P.coord[0],
                               (T*)P.coord[1], (T*)P.coord[2], (cplx_t<T>*)P.extra);
   }
@@ -725,6 +763,13 @@ cudaError_t launch_sort(const SortLayout& L, const Geom& g, int ns, const void* 
   k_subproblems<<<1, 1024, sub_smem, st>>>(P.bin_start, g.nbins, L.maxsub, max_subs, P.sub_bin, P.sub_start,
                                            P.nsub);
   return cudaGetLastError();
+}
+
+template <typename T>
+cudaError_t launch_sort(const SortLayout& L, const Geom& g, int ns, const void* x, const void* y, const void* z,
+                        int64_t M, const SortPtrs& P, cudaStream_t st) {
+  return L.chunk == kRadixThreads * kRadixItemsSmall ? launch_sort_items<T, kRadixItemsSmall>(L, g, ns, x, y, z, M, P, st)
+                                                     : launch_sort_items<T, kRadixItems>(L, g, ns, x, y, z, M, P, st);
 }
 
 template cudaError_t launch_sort<float>(const SortLayout&, const Geom&, int, const void*, const void*, const void*,

@@ -17,9 +17,19 @@ namespace nfx {
 
 constexpr int kT3Blocks = 256;
 
+// Min and max of each of the 2 dim arrays, one launch: blockIdx.y selects the
+// array (dim sources of M, then dim targets of K).
 template <typename T>
-__global__ void k_minmax(const T* __restrict__ a, int64_t n, double* __restrict__ partial) {
+struct T3Arrays {
+  const T* p[6];
+  int64_t n[6];
+};
+
+template <typename T>
+__global__ void k_minmax(T3Arrays<T> arrays, double* __restrict__ partial) {
   __shared__ double s_min[32], s_max[32];
+  const T* __restrict__ a = arrays.p[blockIdx.y];
+  const int64_t n = arrays.n[blockIdx.y];
   double mn = 1e300, mx = -1e300;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     double v = (double)a[i];
@@ -42,12 +52,15 @@ __global__ void k_minmax(const T* __restrict__ a, int64_t n, double* __restrict_
       mn = fmin(mn, s_min[i]);
       mx = fmax(mx, s_max[i]);
     }
-    partial[2 * blockIdx.x] = mn;
-    partial[2 * blockIdx.x + 1] = mx;
+    double* q = partial + ((size_t)blockIdx.y * kT3Blocks + blockIdx.x) * 2;
+    q[0] = mn;
+    q[1] = mx;
   }
 }
 
 // partial: [2*dim arrays][kT3Blocks][2]; arrays 0..dim-1 sources, dim..2dim-1 targets.
+// One warp per array reduces its partials (a single thread reading all of them
+// one after another took 60 us for 2D), then thread 0 writes the scalars.
 // The scalars are computed in the working type T in the reference's order
 // (nufft3.py:258-268, 354-362), with the Python constants rounded to T first
 // as JAX's weak typing does: C = (min + max) / 2, S = max((max - min) / 2,
@@ -57,20 +70,30 @@ __global__ void k_minmax(const T* __restrict__ a, int64_t n, double* __restrict_
 template <typename T>
 __global__ void k_t3_params(const double* __restrict__ partial, int dim, int nf0, int nf1, int nf2,
                             double upsampfac, T3Params* __restrict__ p) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+  __shared__ double s_mn[6], s_mx[6];
+  {
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;  // launched with 2 dim warps
+    const double* q = partial + (size_t)w * kT3Blocks * 2;
+    double lo = 1e300, hi = -1e300;
+    for (int i = lane; i < kT3Blocks; i += 32) {
+      lo = fmin(lo, q[2 * i]);
+      hi = fmax(hi, q[2 * i + 1]);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+      hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+    if (lane == 0) {
+      s_mn[w] = lo;
+      s_mx[w] = hi;
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
   const int nf[3] = {nf0, nf1, nf2};
   for (int d = 0; d < dim; ++d) {
-    T mn[2], mx[2];
-    for (int s = 0; s < 2; ++s) {
-      const double* q = partial + (size_t)(s * dim + d) * kT3Blocks * 2;
-      double a = 1e300, b = -1e300;
-      for (int i = 0; i < kT3Blocks; ++i) {
-        a = fmin(a, q[2 * i]);
-        b = fmax(b, q[2 * i + 1]);
-      }
-      mn[s] = (T)a;
-      mx[s] = (T)b;
-    }
+    const T mn[2] = {(T)s_mn[d], (T)s_mn[dim + d]}, mx[2] = {(T)s_mx[d], (T)s_mx[dim + d]};
     const T C = rn_add(mn[0], mx[0]) / (T)2.0;
     const T D = rn_add(mn[1], mx[1]) / (T)2.0;
     const T half = rn_sub(mx[1], mn[1]) / (T)2.0;
@@ -177,12 +200,16 @@ template <typename T>
 cudaError_t launch_t3_params(int dim, const int nf[3], double upsampfac, const void* const* src, int64_t M,
                              const void* const* tgt, int64_t K, T3Params* params, void* scratch, cudaStream_t st) {
   double* partial = (double*)scratch;
+  T3Arrays<T> arrays{};
   for (int d = 0; d < dim; ++d) {
-    k_minmax<T><<<kT3Blocks, 256, 0, st>>>((const T*)src[d], M, partial + (size_t)d * kT3Blocks * 2);
-    k_minmax<T><<<kT3Blocks, 256, 0, st>>>((const T*)tgt[d], K, partial + (size_t)(dim + d) * kT3Blocks * 2);
+    arrays.p[d] = (const T*)src[d];
+    arrays.n[d] = M;
+    arrays.p[dim + d] = (const T*)tgt[d];
+    arrays.n[dim + d] = K;
   }
-  k_t3_params<T><<<1, 32, 0, st>>>(partial, dim, nf[0], dim > 1 ? nf[1] : 1, dim > 2 ? nf[2] : 1, upsampfac,
-                                   params);
+  k_minmax<T><<<dim3(kT3Blocks, 2 * dim), 256, 0, st>>>(arrays, partial);
+  k_t3_params<T><<<1, 64 * dim, 0, st>>>(partial, dim, nf[0], dim > 1 ? nf[1] : 1, dim > 2 ? nf[2] : 1, upsampfac,
+                                         params);
   return cudaGetLastError();
 }
 
