@@ -234,6 +234,18 @@ int nfx_nufft2(const nfx_opts* opts, const int n_modes[3], const void* x, const 
                const void* f_in, int n_trans, int fft_sign, const void* fac1, const void* fac2, const void* fac3,
                void* fw, void* c_out, void* workspace, size_t workspace_bytes, void* stream);
 
+/* The steps of those pipelines around an already sorted point set, one host call
+ * each: nfx_spread_to_modes = nfx_spread_sorted, nfx_fft, nfx_deconv_shuffle (a
+ * type 1 after its sort); nfx_modes_to_grid = nfx_deconv_pad, nfx_fft (a type 2
+ * before its nfx_interp_sorted).  Arguments, results and errors are theirs; as
+ * nfx_fft they refuse a capturing stream. */
+int nfx_spread_to_modes(const nfx_opts* opts, const int n_modes[3], const void* x, const void* y, const void* z,
+                        int64_t M, const void* c, int n_trans, int fft_sign, const void* fac1, const void* fac2,
+                        const void* fac3, void* fw, void* f_out, const void* workspace, size_t workspace_bytes,
+                        void* stream);
+int nfx_modes_to_grid(int precision, int dim, const int nf[3], const int n_modes[3], const void* f_in, int n_trans,
+                      int fft_sign, const void* fac1, const void* fac2, const void* fac3, void* fw, void* stream);
+
 /* ---- batching: many problems in one launch --------------------------------
  * No counterpart in the reference (nufftax vmaps one problem's strengths).
  * Each problem has its own points, fine grid, tiling and sort workspace; the

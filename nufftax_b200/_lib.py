@@ -140,6 +140,10 @@ _SIGNATURES = {
                     _vp, _vp, c_size_t, _vp], c_int),
     "nfx_nufft2": ([POINTER(NfxOpts), POINTER(c_int), _vp, _vp, _vp, c_int64, _vp, c_int, c_int, _vp, _vp, _vp, _vp,
                     _vp, _vp, c_size_t, _vp], c_int),
+    "nfx_spread_to_modes": ([POINTER(NfxOpts), POINTER(c_int), _vp, _vp, _vp, c_int64, _vp, c_int, c_int, _vp, _vp,
+                             _vp, _vp, _vp, _vp, c_size_t, _vp], c_int),
+    "nfx_modes_to_grid": ([c_int, c_int, POINTER(c_int), POINTER(c_int), _vp, c_int, c_int, _vp, _vp, _vp, _vp, _vp],
+                          c_int),
     "nfx_fft_cache_clear": ([], c_int),
     "nfx_fft_cache_limit": ([c_int], c_int),
     "nfx_batch_info_get": ([POINTER(NfxOpts), c_int, POINTER(NfxBatchProblem), c_int, POINTER(NfxBatchInfo)], c_int),

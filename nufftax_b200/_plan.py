@@ -8,6 +8,7 @@ memory and the current stream; all arithmetic happens in the CUDA library.
 from __future__ import annotations
 
 import collections
+import contextlib
 import threading
 import ctypes
 from ctypes import byref, c_int, c_size_t, c_void_p
@@ -17,8 +18,9 @@ import numpy as np
 import torch
 
 from . import _lib
-from .kernel import KernelParams, deconv_factors
-from .profiling import span
+from .grid import compute_grid_size
+from .kernel import KernelParams, compute_kernel_params, deconv_factors
+from .profiling import recording, span
 
 _REAL = {_lib.NFX_F32: torch.float32, _lib.NFX_F64: torch.float64}
 _CPLX = {_lib.NFX_F32: torch.complex64, _lib.NFX_F64: torch.complex128}
@@ -49,6 +51,16 @@ def stream_of(device: torch.device) -> int:
     if _raw_stream is not None:
         return _raw_stream(device.index if device.index is not None else torch.cuda.current_device())
     return torch.cuda.current_stream(device).cuda_stream
+
+
+_no_switch = contextlib.nullcontext()
+
+
+def on_device(device: torch.device):
+    """torch.cuda.device(device), skipped when it is current already."""
+    if device.index is not None and torch._C._cuda_getDevice() == device.index:
+        return _no_switch
+    return torch.cuda.device(device)
 
 
 def ptr(t: torch.Tensor | None):
@@ -116,7 +128,9 @@ class PointSort:
     """Bin-sorted non-uniform points on one fine grid."""
 
     def __init__(self, coords: Sequence[torch.Tensor], nf: Sequence[int], kp: KernelParams, prenorm: bool,
-                 tile=None, max_subproblem: int = 0, modes=(0, 0)):
+                 tile=None, max_subproblem: int = 0, modes=(0, 0), opts: _lib.NfxOpts | None = None):
+        """opts: the library options of (precision, nf, kp, prenorm, tile, ..) when
+        the caller already has them (copied)."""
         self.dim = len(coords)
         if self.dim not in (1, 2, 3) or len(nf) != self.dim:
             raise ValueError("coords and nf must have 1, 2 or 3 axes")
@@ -131,7 +145,8 @@ class PointSort:
         self.nf = tuple(int(n) for n in nf)
         self.kp = kp
         self.prenorm = prenorm
-        self.opts = make_opts(self.precision, self.nf, kp, prenorm, tile, max_subproblem, modes)
+        self.opts = (make_opts(self.precision, self.nf, kp, prenorm, tile, max_subproblem, modes) if opts is None
+                     else _lib.NfxOpts.from_buffer_copy(opts))
         lib = _lib.load()
         nbytes = c_size_t(0)
         _lib.check(lib.nfx_sort_workspace_bytes(byref(self.opts), self.M, byref(nbytes)), "nfx_sort_workspace_bytes")
@@ -140,7 +155,7 @@ class PointSort:
         self.stream = stream_of(self.device)  # the stream the sort ran on (and the workspace belongs to)
         self._src = None
         launches = lambda: sort_launches(self.opts, self.M)  # noqa: E731 (evaluated only when recording)
-        with torch.cuda.device(self.device), span("nfx_sort_points", self.device, launches):
+        with on_device(self.device), span("nfx_sort_points", self.device, launches):
             _lib.check(lib.nfx_sort_points(byref(self.opts), *self._xyz(), self.M, ptr(self.ws), self.ws_bytes,
                                            c_void_p(stream_of(self.device))), "nfx_sort_points")
             # marks the sort's completion on its stream: a user on another stream
@@ -163,7 +178,7 @@ class PointSort:
 
     def _call(self, name: str, *args):
         lib = _lib.load()
-        with torch.cuda.device(self.device), span(name, self.device, 1 if self.M > 0 else 0):
+        with on_device(self.device), span(name, self.device, 1 if self.M > 0 else 0):
             _lib.check(getattr(lib, name)(byref(self.opts), *self._xyz(), self.M, *args, ptr(self.ws), self.ws_bytes,
                                           c_void_p(stream_of(self.device))), name)
 
@@ -267,7 +282,7 @@ class _SortCache:
         self._cap: "collections.OrderedDict[tuple, PointSort]" = collections.OrderedDict()
         self._lock = threading.Lock()
 
-    def _get_captured(self, coords, nf, kp, prenorm, key) -> PointSort:
+    def _get_captured(self, coords, nf, kp, prenorm, key, opts) -> PointSort:
         dev = coords[0].device
         s = stream_of(dev)
         cid = ctypes.c_ulonglong(0)
@@ -279,7 +294,7 @@ class _SortCache:
             if hit.stream != s:
                 torch.cuda.current_stream(dev).wait_event(hit.ready)
             return hit
-        ps = PointSort(coords, nf, kp, prenorm)
+        ps = PointSort(coords, nf, kp, prenorm, opts=opts)
         ps._src = list(coords)
         with self._lock:
             self._cap[ckey] = ps
@@ -287,11 +302,12 @@ class _SortCache:
                 self._cap.popitem(last=False)
         return ps
 
-    def get(self, coords, nf, kp, prenorm) -> PointSort:
+    def get(self, coords, nf, kp, prenorm, opts: _lib.NfxOpts | None = None) -> PointSort:
+        """The sort of `coords` on the grid, cached or new; opts as PointSort's."""
         key = tuple((id(c), c.data_ptr(), c._version, c.dtype, c.shape[0]) for c in coords) + (
             tuple(nf), kp.nspread, float(kp.beta), float(kp.c), bool(prenorm))
         if torch.cuda.is_current_stream_capturing():
-            return self._get_captured(coords, nf, kp, prenorm, key)
+            return self._get_captured(coords, nf, kp, prenorm, key, opts)
         if self.enabled:
             with self._lock:
                 hit = self._d.get(key)
@@ -306,7 +322,7 @@ class _SortCache:
                     cur.wait_event(hit.ready)
                     hit.ws.record_stream(cur)
                 return hit
-        ps = PointSort(coords, nf, kp, prenorm)
+        ps = PointSort(coords, nf, kp, prenorm, opts=opts)
         ps._src = list(coords)
         if self.enabled:
             with self._lock:
@@ -351,13 +367,93 @@ def factors(nf: int, n_modes: int, kp: KernelParams, precision: int, device: tor
     return t
 
 
+class TransformPlan:
+    """What every call of one transform shape needs and none changes: kernel,
+    grid, library options (coordinates of the transforms, prenorm), mode and grid
+    extents, deconvolution factors on the device.  Holds no points and no
+    workspace."""
+
+    __slots__ = ("kp", "nf", "n_modes", "dim", "precision", "device", "opts", "nf3", "nm3", "facs", "fac_ptrs",
+                 "grid_shape", "mode_shape")
+
+    def __init__(self, n_modes, eps, upsampfac, precision, device):
+        self.n_modes = tuple(n_modes)
+        self.dim = len(self.n_modes)
+        self.kp = compute_kernel_params(eps, upsampfac)
+        self.nf = tuple(compute_grid_size(n, upsampfac, self.kp.nspread) for n in self.n_modes)
+        self.precision = precision
+        self.device = device
+        self.opts = make_opts(precision, self.nf, self.kp, True)
+        self.nf3 = _lib.int3c(self.nf)
+        self.nm3 = _lib.int3c(self.n_modes)
+        self.facs = _facs(self.nf, self.n_modes, self.kp, precision, device)
+        self.fac_ptrs = [ptr(f) for f in self.facs]
+        self.grid_shape = tuple(reversed(self.nf))
+        self.mode_shape = tuple(reversed(self.n_modes))
+
+    def sort(self, coords) -> PointSort:
+        return sort_cache.get(coords, self.nf, self.kp, True, self.opts)
+
+    def type1(self, ps: PointSort, c: torch.Tensor, sign: int) -> torch.Tensor:
+        """Strengths (n_trans, M) at sorted points -> modes: spread, FFT, deconvolve."""
+        c = ps._check_strengths(c)
+        if recording() or torch.cuda.is_current_stream_capturing():
+            # call by call: each is timed, and a captured FFT takes its own work area
+            fw = ps.spread(c)
+            fft_inplace(fw, self.dim, sign)
+            return deconv_shuffle(fw, self.n_modes, self.kp)
+        nt = c.shape[0]
+        fw = torch.empty((nt,) + self.grid_shape, dtype=c.dtype, device=self.device)
+        out = torch.empty((nt,) + self.mode_shape, dtype=c.dtype, device=self.device)
+        f = self.fac_ptrs
+        with on_device(self.device):
+            _lib.check(_lib.load().nfx_spread_to_modes(
+                byref(ps.opts), self.nm3, *ps._xyz(), ps.M, c.data_ptr(), nt, sign, f[0], f[1], f[2], fw.data_ptr(),
+                out.data_ptr(), ps.ws.data_ptr(), ps.ws_bytes, stream_of(self.device)), "nfx_spread_to_modes")
+        return out
+
+    def type2_grid(self, f: torch.Tensor, sign: int) -> torch.Tensor:
+        """Modes (n_trans, ..) -> the fine grid to interpolate: deconvolve, zero-pad, FFT."""
+        f = f.contiguous()
+        if recording() or torch.cuda.is_current_stream_capturing():
+            return fft_inplace(deconv_pad(f, self.nf, self.kp), self.dim, sign)
+        nt = f.shape[0]
+        fw = torch.empty((nt,) + self.grid_shape, dtype=f.dtype, device=self.device)
+        q = self.fac_ptrs
+        with on_device(self.device):
+            _lib.check(_lib.load().nfx_modes_to_grid(
+                self.precision, self.dim, self.nf3, self.nm3, f.data_ptr(), nt, sign, q[0], q[1], q[2], fw.data_ptr(),
+                stream_of(self.device)), "nfx_modes_to_grid")
+        return fw
+
+
+_plan_cache: dict = {}
+_plan_lock = threading.Lock()
+
+
+def transform_plan(n_modes, eps, upsampfac, precision, device) -> TransformPlan:
+    """The shared plan of one transform shape on one device (at most 1024 kept)."""
+    key = (n_modes, eps, upsampfac, precision, device.index)
+    with _plan_lock:
+        pl = _plan_cache.get(key)
+    if pl is None:
+        pl = TransformPlan(n_modes, eps, upsampfac, precision, device)
+        with _plan_lock:
+            if len(_plan_cache) >= 1024:
+                _plan_cache.clear()
+            _plan_cache[key] = pl
+    return pl
+
+
 def clear_caches() -> None:
-    """Drop cached point sorts, deconvolution factors and cuFFT plans.
+    """Drop cached point sorts, transform plans, deconvolution factors and cuFFT plans.
 
     Enqueued deconvolutions (a server's requests in flight, work on any stream)
     may still read the factor tensors, so every device that holds one is
     synchronised before they are dropped."""
     sort_cache.clear()
+    with _plan_lock:
+        _plan_cache.clear()
     with _fac_lock:
         devs = {t.device for t in _fac_cache.values()}
         for d in devs:
@@ -374,7 +470,7 @@ def fft_inplace(fw: torch.Tensor, dim: int, sign: int) -> torch.Tensor:
     precision = precision_of(fw.dtype)
     nf = tuple(reversed(fw.shape[-dim:]))
     lib = _lib.load()
-    with torch.cuda.device(fw.device), span("nfx_fft", fw.device, 0):
+    with on_device(fw.device), span("nfx_fft", fw.device, 0):
         if torch.cuda.is_current_stream_capturing():
             # a captured FFT keeps its work area: take one from the graph's pool
             nbytes = c_size_t(0)
@@ -402,7 +498,7 @@ def deconv_shuffle(fw_hat: torch.Tensor, n_modes: Sequence[int], kp: KernelParam
     fs = _facs(nf, n_modes, kp, precision, fw_hat.device)
     out = torch.empty((fw_hat.shape[0],) + tuple(reversed(n_modes)), dtype=fw_hat.dtype, device=fw_hat.device)
     lib = _lib.load()
-    with torch.cuda.device(fw_hat.device), span("nfx_deconv_shuffle", fw_hat.device):
+    with on_device(fw_hat.device), span("nfx_deconv_shuffle", fw_hat.device):
         _lib.check(lib.nfx_deconv_shuffle(precision, dim, _lib.int3c(nf), _lib.int3c(n_modes), ptr(fs[0]), ptr(fs[1]),
                                           ptr(fs[2]), ptr(fw_hat), ptr(out), int(fw_hat.shape[0]),
                                           c_void_p(stream_of(fw_hat.device))), "nfx_deconv_shuffle")
@@ -419,7 +515,7 @@ def deconv_pad(f: torch.Tensor, nf: Sequence[int], kp: KernelParams, out: torch.
     if out is None:
         out = torch.empty((f.shape[0],) + tuple(reversed(nf)), dtype=f.dtype, device=f.device)
     lib = _lib.load()
-    with torch.cuda.device(f.device), span("nfx_deconv_pad", f.device):
+    with on_device(f.device), span("nfx_deconv_pad", f.device):
         _lib.check(lib.nfx_deconv_pad(precision, dim, _lib.int3c(nf), _lib.int3c(n_modes), ptr(fs[0]), ptr(fs[1]),
                                       ptr(fs[2]), ptr(f), ptr(out), int(f.shape[0]), c_void_p(stream_of(f.device))),
                    "nfx_deconv_pad")

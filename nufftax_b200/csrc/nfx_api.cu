@@ -485,9 +485,55 @@ struct Prepared {
   SortLayout L;
 };
 
+// Resolving options (default tiles, the pitch search, the sort layout) costs 5 to
+// 15 us of host time, and a transform's calls repeat it for the same options and
+// M: each thread keeps its last few answers, by value.  Only successes are kept.
+struct ResolvedOpts {
+  nfx_opts in;
+  int64_t M;
+  Prepared P;
+};
+
+static bool same_opts(const nfx_opts& a, const nfx_opts& b) {
+  bool same = a.precision == b.precision && a.dim == b.dim && a.nspread == b.nspread && a.beta == b.beta &&
+              a.kc == b.kc && a.prenorm == b.prenorm && a.max_subproblem == b.max_subproblem &&
+              a.spread_mode == b.spread_mode && a.interp_mode == b.interp_mode;
+  for (int d = 0; d < 3; ++d) same = same && a.nf[d] == b.nf[d] && a.tile[d] == b.tile[d];
+  return same;
+}
+
+// Resolved options, geometry and sort layout; *key_ok: key_fits (which also sets
+// the error message).
+static int resolve_cached(const nfx_opts* in, int64_t M, Prepared& P, bool* key_ok) {
+  constexpr int kKeep = 8;
+  static thread_local ResolvedOpts kept[kKeep];
+  static thread_local int n_kept = 0, next = 0;
+  if (in != nullptr) {
+    for (int i = 0; i < n_kept; ++i) {
+      if (kept[i].M == M && same_opts(kept[i].in, *in)) {
+        P = kept[i].P;
+        *key_ok = true;
+        return NFX_OK;
+      }
+    }
+  }
+  const int st = resolve_opts(in, P.o);
+  if (st != NFX_OK) return st;
+  fill_geom(&P.o, P.g);
+  make_layout(P.o, P.g, M, P.L);
+  *key_ok = key_fits(P.L);
+  if (*key_ok) {
+    kept[next] = ResolvedOpts{*in, M, P};
+    next = (next + 1) % kKeep;
+    n_kept = n_kept < kKeep ? n_kept + 1 : kKeep;
+  }
+  return NFX_OK;
+}
+
 static int prepare(const nfx_opts* in, int64_t M, const void* x, const void* y, const void* z, const void* ws,
                    size_t ws_bytes, Prepared& P) {
-  int st = resolve_opts(in, P.o);
+  bool key_ok = false;
+  int st = resolve_cached(in, M, P, &key_ok);
   if (st != NFX_OK) return st;
   if (M < 0 || M > (int64_t)INT32_MAX - 1) {
     set_error("M must be in [0, 2^31 - 2]");
@@ -501,9 +547,10 @@ static int prepare(const nfx_opts* in, int64_t M, const void* x, const void* y, 
         return NFX_ERR_INVALID;
       }
   }
-  fill_geom(&P.o, P.g);
-  make_layout(P.o, P.g, M, P.L);
-  if (!key_fits(P.L)) return NFX_ERR_UNSUPPORTED;
+  if (!key_ok) {
+    key_fits(P.L);  // the message
+    return NFX_ERR_UNSUPPORTED;
+  }
   if (ws == nullptr || ws_bytes < P.L.total) {
     set_error("workspace too small: need " + std::to_string(P.L.total) + " bytes");
     return NFX_ERR_WORKSPACE;
@@ -1077,16 +1124,18 @@ int nfx_default_tiles(nfx_opts* opts) {
 }
 
 int nfx_sort_workspace_bytes(const nfx_opts* opts, int64_t M, size_t* bytes) {
-  Prepared P;
-  int st = resolve_opts(opts, P.o);
-  if (st != NFX_OK) return st;
   if (M < 0 || bytes == nullptr) {
+    nfx_opts o;
+    int st = resolve_opts(opts, o);
+    if (st != NFX_OK) return st;
     set_error("M < 0 or bytes is NULL");
     return NFX_ERR_INVALID;
   }
-  fill_geom(&P.o, P.g);
-  make_layout(P.o, P.g, M, P.L);
-  if (!key_fits(P.L)) return NFX_ERR_UNSUPPORTED;
+  Prepared P;
+  bool key_ok = false;
+  int st = resolve_cached(opts, M, P, &key_ok);
+  if (st != NFX_OK) return st;
+  if (!key_ok) return NFX_ERR_UNSUPPORTED;
   *bytes = P.L.total;
   return NFX_OK;
 }
@@ -1254,6 +1303,28 @@ int nfx_nufft2(const nfx_opts* opts, const int n_modes[3], const void* x, const 
   if (st == NFX_OK) st = nfx_fft(opts->precision, opts->dim, opts->nf, n_trans, fw, fft_sign, stream);
   if (st == NFX_OK) st = nfx_sort_points(opts, x, y, z, M, ws, ws_bytes, stream);
   if (st == NFX_OK) st = nfx_interp_sorted(opts, x, y, z, M, fw, n_trans, c_out, ws, ws_bytes, stream);
+  return st;
+}
+
+int nfx_spread_to_modes(const nfx_opts* opts, const int n_modes[3], const void* x, const void* y, const void* z,
+                        int64_t M, const void* c, int n_trans, int fft_sign, const void* fac1, const void* fac2,
+                        const void* fac3, void* fw, void* f_out, const void* ws, size_t ws_bytes, void* stream) {
+  if (opts == nullptr || n_modes == nullptr) {
+    set_error("nfx_spread_to_modes: opts or n_modes is NULL");
+    return NFX_ERR_INVALID;
+  }
+  int st = nfx_spread_sorted(opts, x, y, z, M, c, n_trans, fw, ws, ws_bytes, stream);
+  if (st == NFX_OK) st = nfx_fft(opts->precision, opts->dim, opts->nf, n_trans, fw, fft_sign, stream);
+  if (st == NFX_OK)
+    st = nfx_deconv_shuffle(opts->precision, opts->dim, opts->nf, n_modes, fac1, fac2, fac3, fw, f_out, n_trans,
+                            stream);
+  return st;
+}
+
+int nfx_modes_to_grid(int precision, int dim, const int nf[3], const int n_modes[3], const void* f_in, int n_trans,
+                      int fft_sign, const void* fac1, const void* fac2, const void* fac3, void* fw, void* stream) {
+  int st = nfx_deconv_pad(precision, dim, nf, n_modes, fac1, fac2, fac3, f_in, fw, n_trans, stream);
+  if (st == NFX_OK) st = nfx_fft(precision, dim, nf, n_trans, fw, fft_sign, stream);
   return st;
 }
 

@@ -2,6 +2,7 @@
 
 from __future__ import annotations
 
+import functools
 import math
 
 import numpy as np
@@ -25,8 +26,18 @@ def next_smooth_int(n: int) -> int:
 
 
 def compute_grid_size(n_modes: int, upsampfac: float, nspread: int) -> int:
-    """nf = smooth(max(ceil(upsampfac * n_modes), 2 * nspread)) (grid.py:36-58)."""
+    """nf = smooth(max(ceil(upsampfac * n_modes), 2 * nspread)) (grid.py:36-58).
+    Answers for plain Python numbers are kept."""
+    if type(n_modes) is int and type(upsampfac) is float and type(nspread) is int:
+        return _grid_size_kept(n_modes, upsampfac, nspread)
+    return _grid_size(n_modes, upsampfac, nspread)
+
+
+def _grid_size(n_modes, upsampfac, nspread) -> int:
     return next_smooth_int(max(int(math.ceil(upsampfac * n_modes)), 2 * nspread))
+
+
+_grid_size_kept = functools.lru_cache(maxsize=4096)(_grid_size)
 
 
 def _next_smooth_even(n: int) -> int:

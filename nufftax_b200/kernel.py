@@ -5,6 +5,7 @@ Host-side scalars: these run once per plan, in float64, and feed the CUDA kernel
 
 from __future__ import annotations
 
+import functools
 import math
 from typing import NamedTuple
 
@@ -25,8 +26,14 @@ def compute_kernel_params(tol: float, upsampfac: float = 2.0, max_nspread: int =
 
     nspread = ceil(-log10 tol + 1), clamped to [2, max_nspread] and rounded up to
     even; beta = pi sqrt(ns^2 / sigma^2 (sigma - 1/2)^2 - 0.8) (2.3 ns if the root
-    is not real); c = 4 / ns^2.
+    is not real); c = 4 / ns^2.  Answers for plain Python numbers are kept.
     """
+    if type(tol) is float and type(upsampfac) is float and type(max_nspread) is int:
+        return _kernel_params_kept(tol, upsampfac, max_nspread)
+    return _kernel_params(tol, upsampfac, max_nspread)
+
+
+def _kernel_params(tol, upsampfac, max_nspread) -> KernelParams:
     log_tol = -math.log10(max(tol, 1e-16))
     nspread = int(math.ceil(log_tol + 1))
     nspread = max(2, min(nspread, max_nspread))
@@ -36,6 +43,9 @@ def compute_kernel_params(tol: float, upsampfac: float = 2.0, max_nspread: int =
     inner = (nspread**2) / (sigma**2) * (sigma - 0.5) ** 2 - 0.8
     beta = math.pi * math.sqrt(inner) if inner > 0 else 2.3 * nspread
     return KernelParams(nspread=nspread, beta=beta, c=4.0 / (nspread**2), upsampfac=upsampfac)
+
+
+_kernel_params_kept = functools.lru_cache(maxsize=1024)(_kernel_params)
 
 
 def es_kernel(z: np.ndarray, beta: float, c: float) -> np.ndarray:

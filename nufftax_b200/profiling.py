@@ -52,6 +52,11 @@ def record(only=None):
         _state.rec = prev
 
 
+def recording() -> bool:
+    """Whether a `record()` is active on this thread."""
+    return getattr(_state, "rec", None) is not None
+
+
 class span:
     """Brackets one library call with CUDA events while a `record()` is active
     on this thread; otherwise does nothing (a plain object, no generator, so

@@ -45,8 +45,8 @@ import torch
 import torch.autograd.forward_ad as _fwad
 
 from . import _lib
-from ._plan import (_facs, complex_dtype, deconv_pad, deconv_shuffle, fft_inplace, make_opts, precision_of, ptr,
-                    real_dtype, sort_cache, sort_launches, stream_of)
+from ._plan import (_facs, complex_dtype, make_opts, on_device, precision_of, ptr, real_dtype, sort_launches,
+                    stream_of, transform_plan)
 from .profiling import span
 from .grid import compute_grid_size
 from .kernel import compute_kernel_params
@@ -159,50 +159,37 @@ def _bdim_front(t, bdim, B):
 # transforms can unwrap the inputs level by level.
 # ---------------------------------------------------------------------------
 def _type1_forward(c2, n_modes, eps, isign, uf, coords):
-    dim = len(coords)
-    kp = compute_kernel_params(eps, uf)
-    nf = tuple(compute_grid_size(n, uf, kp.nspread) for n in n_modes)
-    ps = sort_cache.get(list(coords), nf, kp, prenorm=True)
-    fw = ps.spread(c2)
-    fft_inplace(fw, dim, _fft_sign_type1(isign))
-    return deconv_shuffle(fw, n_modes, kp)
+    pl = transform_plan(n_modes, eps, uf, precision_of(c2.dtype), c2.device)
+    return pl.type1(pl.sort(coords), c2, _fft_sign_type1(isign))
 
 
 def _type1_coord_grad(c2, G, n_modes, eps, isign, uf_t, need_c, need_x, coords):
     """(dc or None, [dx_d or None]) of f = type 1 (c2 at coords) for the mode
     cotangent G: G deconvolved, zero-padded and transformed back onto the fine
     grid, then one fused ES-derivative pass over the points."""
-    dim = len(coords)
-    kp = compute_kernel_params(eps, uf_t)
-    nf = tuple(compute_grid_size(n, uf_t, kp.nspread) for n in n_modes)
-    H = deconv_pad(G.contiguous(), nf, kp)
-    fft_inplace(H, dim, -_fft_sign_type1(isign))
-    ps = sort_cache.get(list(coords), nf, kp, prenorm=True)
-    return ps.spread_grad(c2.contiguous(), H, need_c, need_x)
+    pl = transform_plan(n_modes, eps, uf_t, precision_of(G.dtype), G.device)
+    H = pl.type2_grid(G, -_fft_sign_type1(isign))
+    return pl.sort(coords).spread_grad(c2.contiguous(), H, need_c, need_x)
 
 
-def _type2_grid(f2, n_modes, eps, isign, uf, dim):
-    kp = compute_kernel_params(eps, uf)
-    nf = tuple(compute_grid_size(n, uf, kp.nspread) for n in n_modes)
-    fw = deconv_pad(f2, nf, kp)
-    fft_inplace(fw, dim, _fft_sign_type2(isign))
-    return fw, nf, kp
+def _type2_plan(f2, eps, uf):
+    n_modes = tuple(int(v) for v in reversed(f2.shape[1:]))
+    return transform_plan(n_modes, eps, uf, precision_of(f2.dtype), f2.device)
 
 
 def _type2_forward(f2, eps, isign, uf, coords):
-    dim = len(coords)
-    n_modes = tuple(int(v) for v in reversed(f2.shape[1:]))
-    fw, nf, kp = _type2_grid(f2, n_modes, eps, isign, uf, dim)
-    return sort_cache.get(list(coords), nf, kp, prenorm=True).interp(fw)
+    pl = _type2_plan(f2, eps, uf)
+    fw = pl.type2_grid(f2, _fft_sign_type2(isign))
+    return pl.sort(coords).interp(fw)
 
 
 def _type2_coord_grad(f2, G, n_modes, eps, isign, uf, need_x, coords):
     """[dx_d or None] of c = type 2 (f2 at coords) for the point cotangent G:
     the forward fine grid again (deconvolve + FFT), then the ES-derivative
     interpolation on it."""
-    dim = len(coords)
-    fw, nf, kp = _type2_grid(f2.contiguous(), n_modes, eps, isign, uf, dim)
-    return sort_cache.get(list(coords), nf, kp, prenorm=True).interp_grad(fw, G.contiguous(), need_x)
+    pl = _type2_plan(f2, eps, uf)
+    fw = pl.type2_grid(f2, _fft_sign_type2(isign))
+    return pl.sort(coords).interp_grad(fw, G.contiguous(), need_x)
 
 
 def _split_stack(F, nt, first):
@@ -504,10 +491,10 @@ def _type3_forward(src: list[torch.Tensor], c2: torch.Tensor, tgt: list[torch.Te
     src = [a.contiguous() for a in src]
     tgt = [a.contiguous() for a in tgt]
     c2 = c2.contiguous()
-    # our kernels: min / max per array, the scalars, both sorts, spread, zero-pad, interp
-    launches = lambda: (2 * dim + 1 + sort_launches(opts, M, type3=True) + 2  # noqa: E731 (evaluated only when recording)
+    # our kernels: min / max of every array, the scalars, both sorts, spread, zero-pad, interp
+    launches = lambda: (2 + sort_launches(opts, M, type3=True) + 2  # noqa: E731 (evaluated only when recording)
                         + sort_launches(make_opts(precision, nf_in, kp, prenorm=True), K, type3=True) + 1)
-    with torch.cuda.device(dev), span("nfx_nufft3", dev, launches):
+    with on_device(dev), span("nfx_nufft3", dev, launches):
         _lib.check(lib.nfx_nufft3(byref(opts), _lib.int3c(nf_in), float(uf), int(isign), parr(src), M, ptr(c2), nt,
                                   parr(tgt), K, ptr(facs[0]), ptr(facs[1]), ptr(facs[2]), ptr(out), ptr(ws),
                                   ws.numel(), c_void_p(stream_of(dev))), "nfx_nufft3")
