@@ -94,12 +94,16 @@ constexpr int64_t kRadixSmallM = 148 * 2 * kRadixThreads * kRadixItemsSmall;  //
 // One CTA per chunk of consecutive points: K = bin << cbits | cell
 // for every point, and the chunk's histogram of digit 0 as row `chunk` of
 // counts (chunk-major, so the row is one coalesced write).
+// A thread takes kKeyItems points, so a 4096-point chunk has 1024 threads: with
+// 256 threads of 16 points each, a chunk's folds ran one after another at two
+// warps a scheduler (524 k points, one chunk an SM: 11 us).
 // T3: the points are type-3 sources or targets (Geom::t3_mode), a separate
 // instantiation so the common kernel carries no type-3 code.
 // f[d] (nullptr: not wanted): every point's folded coordinates in input order,
 // the payload the scatter passes then carry into sorted order.
-template <typename T, int DIM, bool T3, int ITEMS>
-__global__ void __launch_bounds__(kRadixThreads, ITEMS > 4 ? 4 : 1) k_sort_keys(const T* __restrict__ x, const T* __restrict__ y,
+constexpr int kKeyItems = 4;
+template <typename T, int DIM, bool T3>
+__global__ void __launch_bounds__(1024) k_sort_keys(const T* __restrict__ x, const T* __restrict__ y,
                                                             const T* __restrict__ z, int M, Geom g, int ns_half,
                                                             int cbits, int dbits, int* __restrict__ K,
                                                             int* __restrict__ counts, T* __restrict__ f0,
@@ -109,19 +113,19 @@ __global__ void __launch_bounds__(kRadixThreads, ITEMS > 4 ? 4 : 1) k_sort_keys(
   const int mask = B - 1;
   for (int i = threadIdx.x; i < B; i += blockDim.x) s_h[i] = 0;
   __syncthreads();
-  const int c0 = blockIdx.x * (kRadixThreads * ITEMS);
+  const int c0 = blockIdx.x * blockDim.x * kKeyItems;
   const T* cs[3] = {x, y, z};
   // all coordinate loads first, so they are in flight together
-  T cv[ITEMS][DIM];
+  T cv[kKeyItems][DIM];
 #pragma unroll
-  for (int u = 0; u < ITEMS; ++u) {
-    const int p = c0 + u * kRadixThreads + threadIdx.x;
+  for (int u = 0; u < kKeyItems; ++u) {
+    const int p = c0 + u * blockDim.x + threadIdx.x;
 #pragma unroll
     for (int d = 0; d < DIM; ++d) cv[u][d] = p < M ? cs[d][p] : (T)0;
   }
 #pragma unroll
-  for (int u = 0; u < ITEMS; ++u) {
-    const int p = c0 + u * kRadixThreads + threadIdx.x;
+  for (int u = 0; u < kKeyItems; ++u) {
+    const int p = c0 + u * blockDim.x + threadIdx.x;
     if (p < M) {
       int kb, kc;
       T xs[DIM];
@@ -708,14 +712,14 @@ static cudaError_t launch_sort_items(const SortLayout& L, const Geom& g, int ns,
     if (e != cudaSuccess) return e;
     const unsigned scan_grid = (unsigned)((B + kScanDigits - 1) / kScanDigits);
     auto keys = g.t3_mode != 0
-                    ? (g.dim == 1 ? k_sort_keys<T, 1, true, ITEMS> : (g.dim == 2 ? k_sort_keys<T, 2, true, ITEMS> : k_sort_keys<T, 3, true, ITEMS>))
-                    : (g.dim == 1 ? k_sort_keys<T, 1, false, ITEMS>
-                                  : (g.dim == 2 ? k_sort_keys<T, 2, false, ITEMS> : k_sort_keys<T, 3, false, ITEMS>));
+                    ? (g.dim == 1 ? k_sort_keys<T, 1, true> : (g.dim == 2 ? k_sort_keys<T, 2, true> : k_sort_keys<T, 3, true>))
+                    : (g.dim == 1 ? k_sort_keys<T, 1, false>
+                                  : (g.dim == 2 ? k_sort_keys<T, 2, false> : k_sort_keys<T, 3, false>));
     // ping-pong so that the last pass writes (keys_sorted, perm[, coord]); the
     // keys kernel writes the input-order coordinates into the buffer the first
     // pass does not write
     void* const* cfirst = (L.npass % 2 == 0) ? P.coord : P.coord_tmp;
-    keys<<<L.nchunks, kRadixThreads, hist_smem, st>>>(
+    keys<<<L.nchunks, L.chunk / kKeyItems, hist_smem, st>>>(
         (const T*)x, (const T*)y, (const T*)z, (int)M, g, ns / 2, L.cbits, L.dbits, P.keys, P.counts,
         carry ? (T*)cfirst[0] : nullptr, carry ? (T*)cfirst[1] : nullptr, carry ? (T*)cfirst[2] : nullptr);
     const int* kin = P.keys;
