@@ -660,10 +660,90 @@ static bool es_poly(int ns, double beta, double kc, EsPoly& out, double* err = n
   return out.deg > 0;
 }
 
+// Double inner weights: Chebyshev interpolation of degree kPolyEvalDegD at its
+// zeros in extended precision, converted to monomials in v.  Accepted when the
+// even / odd form the kernels evaluate in double stays within
+// kPolyDRel * (largest value of that weight) of the extended-precision value on
+// a fine grid: less than the rounding of beta (sqrt(..) - 1) costs the exp/sqrt
+// form (about beta / 2 roundings).
+constexpr double kPolyDRel = 4e-16;
+
+static long double es_phil(long double z, double beta, double kc) {
+  const long double arg = 1.0L - (long double)kc * z * z;
+  return arg >= 0.0L ? std::exp((long double)beta * (std::sqrt(arg) - 1.0L)) : 0.0L;
+}
+
+static bool fit_es_polyd(int ns, double beta, double kc, EsPolyD& out) {
+  constexpr int D = kPolyEvalDegD, n = D + 1;
+  const long double pi = std::acos(-1.0L);
+  EsPolyD P = {};
+  P.deg = D;
+  for (int q = 1; q < ns / 2; ++q) {
+    long double cheb[n] = {0};
+    for (int j = 0; j < n; ++j) {
+      long double acc = 0.0L;
+      for (int k = 0; k < n; ++k) {
+        const long double th = pi * (k + 0.5L) / n;
+        acc += es_phil(q - (std::cos(th) + ns - 1) / 2.0L, beta, kc) * std::cos(j * th);
+      }
+      cheb[j] = (j == 0 ? 1.0L : 2.0L) * acc / n;
+    }
+    // Chebyshev -> monomial: T_{j+1} = 2 v T_j - T_{j-1}
+    long double mono[n] = {0}, t0[n] = {0}, t1[n] = {0}, t2[n];
+    t0[0] = 1.0L;
+    t1[1] = 1.0L;
+    for (int i = 0; i < n; ++i) mono[i] = cheb[0] * t0[i] + cheb[1] * t1[i];
+    for (int j = 2; j < n; ++j) {
+      for (int i = 0; i < n; ++i) t2[i] = (i > 0 ? 2.0L * t1[i - 1] : 0.0L) - t0[i];
+      for (int i = 0; i < n; ++i) {
+        t0[i] = t1[i];
+        t1[i] = t2[i];
+        mono[i] += cheb[j] * t2[i];
+      }
+    }
+    for (int i = 0; i < n; ++i) P.a[q - 1][i] = (double)mono[i];
+    long double worst = 0.0L, largest = 0.0L;
+    for (int t = 0; t <= 500; ++t) {
+      const double v = -1.0 + 2.0 * t / 500.0, u = v * v;
+      double e = P.a[q - 1][D - 1], o = P.a[q - 1][D];
+      for (int d = D - 3; d >= 0; d -= 2) {
+        e = std::fma(e, u, P.a[q - 1][d]);
+        o = std::fma(o, u, P.a[q - 1][d + 1]);
+      }
+      for (int side = -1; side <= 1; side += 2) {
+        const long double ref = es_phil(q - ((long double)(side * v) + ns - 1) / 2.0L, beta, kc);
+        const long double err = std::fabs((long double)std::fma(side * v, o, e) - ref);
+        worst = err > worst ? err : worst;
+        largest = ref > largest ? ref : largest;
+      }
+    }
+    if (!(worst <= kPolyDRel * largest)) return false;
+  }
+  out = P;
+  return ns >= 4;
+}
+
+static void es_polyd(int ns, double beta, double kc, EsPolyD& out) {
+  static std::mutex mu;
+  static std::map<std::tuple<int, double, double>, EsPolyD> cache;
+  std::lock_guard<std::mutex> lk(mu);
+  auto key = std::make_tuple(ns, beta, kc);
+  auto it = cache.find(key);
+  if (it == cache.end()) {
+    EsPolyD P = {};
+    if (!fit_es_polyd(ns, beta, kc, P)) P.deg = 0;
+    it = cache.emplace(key, P).first;
+  }
+  out = it->second;
+}
+
 template <typename T>
 static void attach_poly(PointArgs<T>& a, int ns, double beta, double kc) {
   a.poly.deg = 0;
-  if (std::is_same<T, float>::value) es_poly(ns, beta, kc, a.poly);
+  if constexpr (std::is_same<T, float>::value)
+    es_poly(ns, beta, kc, a.poly);
+  else
+    es_polyd(ns, beta, kc, a.polyd);
 }
 
 template <typename T>
@@ -1421,6 +1501,7 @@ int nfx_batch_upload(const nfx_opts* common, int spread, const nfx_batch_problem
     } else {
       BatchItem<double>* it = (BatchItem<double>*)host.data() + p;
       it->a = make_args<double>(P.g, P.o.beta, P.o.kc, probs[p].M, 1, view(P.L, probs[p].workspace));
+      attach_poly(it->a, P.o.nspread, P.o.beta, P.o.kc);
       if (spread) split_batch_items<double>(P, M_total, it->a);
       it->src = probs[p].src;
       it->dst = probs[p].dst;

@@ -229,6 +229,17 @@ struct EsPoly {
   int deg;  // 0 = not used (exp/sqrt form)
 };
 
+// Polynomial form of the ES weights of one footprint (double path): the weights
+// of the inner cells q = 1 .. ns - 2, in pairs as above (a[q - 1] for q < ns / 2,
+// fitted in extended precision, nfx_api.cu fit_es_polyd).  The first and last
+// weight, whose cells reach the kernel's edge and its square-root singularity,
+// keep the exp/sqrt form.
+constexpr int kPolyEvalDegD = 17;
+struct EsPolyD {
+  double a[7][kPolyEvalDegD + 1];
+  int deg;  // 0 = not used (exp/sqrt form)
+};
+
 // Exact division of a non-negative int n < 2^31 by a fixed divisor d >= 1 as a
 // multiply-high and a shift: with p = 31 + ceil(log2 d) and m = ceil(2^p / d)
 // (which fits in 32 bits), n * m / 2^p = n / d + n e / (d 2^p) for some

@@ -52,13 +52,17 @@ struct PointArgs {
   T beta, kc;
   SortView s;
   EsPoly poly;
+  std::conditional_t<sizeof(T) == 8, EsPolyD, char> polyd;  // double only
 };
 
 // The NS weights of one axis: w[q] = phi(i0 + q - xs).  float with a fitted
 // polynomial: Horner in v = 2 (xs - i0) - (NS - 1) (exact in float: xs - i0 is
 // exact because xs and i0 are within NS of each other and i0 is an integer),
 // degree kPolyEvalDeg, each coefficient a fixed offset in the argument block
-// (an operand of its FMA, no load); otherwise exp/sqrt
+// (an operand of its FMA, no load).  double likewise, but the two edge weights
+// by exp/sqrt: 10 DFMA a weight instead of about 55 double operations, which
+// bound the complex128 kernels (2D, 200 k points, ns 14: spread 97 us, of them
+// about two thirds the 28 weights of a point).  Otherwise exp/sqrt
 // (nufftax/core/kernel.py:79-111).
 template <typename T, int NS>
 __device__ __forceinline__ void axis_weights(const PointArgs<T>& a, int i0, T xs, T* w) {
@@ -87,10 +91,31 @@ __device__ __forceinline__ void axis_weights(const PointArgs<T>& a, int i0, T xs
       w[q] = (T)fmaf(v, o[q], e[q]);
       w[NS - 1 - q] = (T)fmaf(-v, o[q], e[q]);
     }
-  } else {
-#pragma unroll
-    for (int q = 0; q < NS; ++q) w[q] = es_weight(rn_sub((T)(i0 + q), xs), a.beta, a.kc);
+    return;
   }
+  if constexpr (sizeof(T) == 8 && NS >= 4) {
+    if (a.polyd.deg > 0) {
+      static_assert(kPolyEvalDegD % 2 == 1, "odd evaluation degree: E and O of equal length");
+      const double v = 2.0 * (xs - (T)i0) - (double)(NS - 1);
+      const double u = v * v;
+#pragma unroll
+      for (int q = 1; q < NS / 2; ++q) {
+        double e = a.polyd.a[q - 1][kPolyEvalDegD - 1], o = a.polyd.a[q - 1][kPolyEvalDegD];
+#pragma unroll
+        for (int d = kPolyEvalDegD - 3; d >= 0; d -= 2) {
+          e = fma(e, u, a.polyd.a[q - 1][d]);
+          o = fma(o, u, a.polyd.a[q - 1][d + 1]);
+        }
+        w[q] = fma(v, o, e);
+        w[NS - 1 - q] = fma(-v, o, e);
+      }
+      w[0] = es_weight(rn_sub((T)i0, xs), a.beta, a.kc);
+      w[NS - 1] = es_weight(rn_sub((T)(i0 + NS - 1), xs), a.beta, a.kc);
+      return;
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < NS; ++q) w[q] = es_weight(rn_sub((T)(i0 + q), xs), a.beta, a.kc);
 }
 
 __device__ __forceinline__ void bin_origin(const Geom& g, int b, int& o0, int& o1, int& o2) {
@@ -1487,6 +1512,7 @@ PointArgs<T> make_args(const Geom& g, double beta, double kc, int64_t M, int n_t
   a.kc = (T)kc;
   a.s = s;
   a.poly.deg = 0;
+  if constexpr (sizeof(T) == 8) a.polyd.deg = 0;
   return a;
 }
 
