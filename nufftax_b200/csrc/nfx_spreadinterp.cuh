@@ -1104,10 +1104,135 @@ __global__ void __launch_bounds__(NW * 32) k_interp_batch(const BatchItem<T>* __
 }
 
 // ---------------------------------------------------------------------------
+// Gradient pass with one lane group per point (3D; layout as interp_group): lane
+// kx reads footprint column kx of every (ky, kz) once and uses it for the value
+// and all three derivative sums.  A thread per point reads 32 scattered
+// footprints at a time, and the bank conflicts of those were 54 % of its
+// shared-memory wavefronts, which bound it (88 % of that roof).
+// ---------------------------------------------------------------------------
+template <typename T, int NS, int NW>
+__device__ __forceinline__ bool grad_group(const PointArgs<T>& a, const cplx_t<T>* __restrict__ G,
+                                           const cplx_t<T>* __restrict__ V, cplx_t<T>* __restrict__ out_interp,
+                                           T* __restrict__ dx, T* __restrict__ dy, T* __restrict__ dz, int sidx,
+                                           unsigned char* smem_raw, TmaStage& ts) {
+  using CT = cplx_t<T>;
+  constexpr int GL = group_lanes<NS>();
+  constexpr int PPW = 32 / GL;
+  constexpr unsigned kAll = 0xffffffffu;
+  CT* s_tile = reinterpret_cast<CT*>(smem_raw);
+  const Geom& g = a.g;
+  const int row = g.pitch;
+  const int plane = g.pitch * g.pad[1];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int kx = lane % GL;
+  const int leader = lane - kx;
+  const bool col_on = kx < NS;
+  T scale[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) scale[d] = -(T)((double)g.nf[d] / (2.0 * kPi));
+  // the group's first lanes store one output each: the value, then dx, dy, dz
+  T* dout = kx == 1 ? dx : (kx == 2 ? dy : (kx == 3 ? dz : nullptr));
+  const int b = a.s.sub_bin[sidx];
+  const int k0 = a.s.sub_start[sidx];
+  const int k1 = min(k0 + a.s.maxsub, a.s.bin_start[b + 1]);
+  int o[3];
+  bin_origin(g, b, o[0], o[1], o[2]);
+  for (int t = 0; t < a.n_trans; ++t) {
+    __syncthreads();
+    if (!stage_interp_tile<T>(a, o, G, t, s_tile, ts)) return false;
+    __syncthreads();
+    constexpr int kStep = NW * 32;
+    const int kw = k0 + warp * 32;
+    // permutation two rounds ahead, coordinates and V one round ahead
+    int p_cur = round_perm(a.s, kw, k1), p_next = round_perm(a.s, kw + kStep, k1);
+    T x_cur[3];
+    round_coords<T, 3>(a, kw, k1, x_cur);
+    CT v_cur;
+    v_cur.x = v_cur.y = (T)0;
+    if (p_cur >= 0) v_cur = V[(int64_t)t * a.M + p_cur];
+    for (int kb = kw; kb < k1; kb += kStep) {  // warp-uniform
+      const WarpPoints<T> wp = warp_points<T, 3, NS>(a, p_cur, x_cur, o, row, plane);
+      const CT vv = v_cur;
+      p_cur = p_next;
+      p_next = round_perm(a.s, kb + 2 * kStep, k1);
+      round_coords<T, 3>(a, kb + kStep, k1, x_cur);
+      if (p_cur >= 0) v_cur = V[(int64_t)t * a.M + p_cur];
+      const int npts = min(32, k1 - kb);
+#pragma unroll 1
+      for (int j0 = 0; j0 < npts; j0 += PPW) {
+        const int j = j0 + lane / GL;
+        const bool valid = j < npts;
+        const int src = valid ? j : 0;
+        const WarpPoints<T> pt = group_take<T, 3>(wp, src);
+        CT v;
+        v.x = __shfl_sync(kAll, vv.x, src);
+        v.y = __shfl_sync(kAll, vv.y, src);
+        const bool on = col_on && pt.off >= 0;
+        T w[3], dw[3];  // this lane's weight q = kx of each axis, and its derivative
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          es_weight_deriv(rn_sub((T)(pt.i0[d] + kx), pt.xs[d]), a.beta, a.kc, w[d], dw[d]);
+          dw[d] *= scale[d];
+        }
+        // one accumulator pair per z plane: plain and y-differentiated
+        CT acc[NS], accd[NS];
+#pragma unroll
+        for (int kz = 0; kz < NS; ++kz) acc[kz].x = acc[kz].y = accd[kz].x = accd[kz].y = (T)0;
+        const CT* base = s_tile + (on ? pt.off + kx : 0);
+#pragma unroll
+        for (int ky = 0; ky < NS; ++ky) {
+          const T wy = __shfl_sync(kAll, w[1], leader + ky), dwy = __shfl_sync(kAll, dw[1], leader + ky);
+#pragma unroll
+          for (int kz = 0; kz < NS; ++kz) {
+            const CT u = base[kz * plane + ky * row];
+            acc[kz] = fma2(splat2(wy), u, acc[kz]);
+            accd[kz] = fma2(splat2(dwy), u, accd[kz]);
+          }
+        }
+        CT s0, sy, sz;
+        s0.x = s0.y = sy.x = sy.y = sz.x = sz.y = (T)0;
+#pragma unroll
+        for (int kz = 0; kz < NS; ++kz) {
+          const T wz = __shfl_sync(kAll, w[2], leader + kz), dwz = __shfl_sync(kAll, dw[2], leader + kz);
+          s0 = fma2(splat2(wz), acc[kz], s0);
+          sy = fma2(splat2(wz), accd[kz], sy);
+          sz = fma2(splat2(dwz), acc[kz], sz);
+        }
+        // Re(conj(v) * s) = v.x s.x + v.y s.y per column, then summed over the columns
+        T r[5];
+        r[0] = on ? s0.x * w[0] : (T)0;
+        r[1] = on ? s0.y * w[0] : (T)0;
+        r[2] = on ? (v.x * s0.x + v.y * s0.y) * dw[0] : (T)0;
+        r[3] = on ? (v.x * sy.x + v.y * sy.y) * w[0] : (T)0;
+        r[4] = on ? (v.x * sz.x + v.y * sz.y) * w[0] : (T)0;
+#pragma unroll
+        for (int m = GL / 2; m >= 1; m >>= 1) {
+#pragma unroll
+          for (int i = 0; i < 5; ++i) r[i] += __shfl_xor_sync(kAll, r[i], m);
+        }
+        if (valid) {
+          if (kx == 0 && out_interp != nullptr) {
+            CT u;
+            u.x = r[0];
+            u.y = r[1];
+            out_interp[(int64_t)t * a.M + pt.p] = u;
+          }
+          if (dout != nullptr) {
+            const T val = kx == 1 ? r[2] : (kx == 2 ? r[3] : r[4]);
+            dout[pt.p] = t == 0 ? val : dout[pt.p] + val;
+          }
+        }
+      }
+    }
+  }
+  return true;
+}
+
+// ---------------------------------------------------------------------------
 // Gradient pass (see launch_grad in nfx_internal.h)
 // ---------------------------------------------------------------------------
 template <typename T, int DIM, int NS, int NW>
-__global__ void __launch_bounds__(NW * 32) k_grad(PointArgs<T> a, const cplx_t<T>* __restrict__ G,
+__global__ void __launch_bounds__(NW * 32) k_grad(const __grid_constant__ PointArgs<T> a, const cplx_t<T>* __restrict__ G,
                                                   const cplx_t<T>* __restrict__ V, cplx_t<T>* __restrict__ out_interp,
                                                   T* __restrict__ dx, T* __restrict__ dy, T* __restrict__ dz,
                                                   const __grid_constant__ CUtensorMap tmap) {
@@ -1124,6 +1249,19 @@ __global__ void __launch_bounds__(NW * 32) k_grad(PointArgs<T> a, const cplx_t<T
   T* douts[3] = {dx, dy, dz};
   for (int sidx = blockIdx.x; sidx < nsub; sidx += gridDim.x) {
     const int b = a.s.sub_bin[sidx];
+    // 3D, a lane group per point where the bin holds fewer points than cells: a
+    // warp's 32 points are then many cells apart and their footprint reads
+    // conflict.  In denser bins neighbouring threads read nearly the same cells,
+    // and a thread per point is the faster one.  Thread -> group, us, complex64 ns
+    // 8: 8M on 256^3 (0.5 a cell) 2592 -> 2176, 1M on 192x225x256 583 -> 539; but
+    // 4M on 128^3 (1.9 a cell) 881 -> 946, 1M clustered 254 -> 311.  Widths that
+    // fill their lane groups only (ns 6 398 -> 445, complex128 ns 10 315 -> 381).
+    if constexpr (DIM == 3 && (NS == 4 || NS == 8)) {
+      if (a.s.bin_start[b + 1] - a.s.bin_start[b] < g.tile[0] * g.tile[1] * g.tile[2]) {
+        if (!grad_group<T, NS, NW>(a, G, V, out_interp, dx, dy, dz, sidx, smem_raw, ts)) return;
+        continue;
+      }
+    }
     const int k0 = a.s.sub_start[sidx];
     const int k1 = min(k0 + a.s.maxsub, a.s.bin_start[b + 1]);
     int o[3];
