@@ -250,7 +250,8 @@ ALG_BYTES = {
 
 # Per-launch counters of the spread / interp kernels on each point set, from
 # single-step ncu --metrics captures of `bench.py --case radial|clustered --reps 1`
-# (profiles/k_spread_interp_2d_counters.md): DRAM bytes (dram__bytes_read.sum +
+# (profiles/window_spread.md for the spread, on sets of the same distributions;
+# profiles/k_spread_interp_2d_counters.md for the interpolation): DRAM bytes (dram__bytes_read.sum +
 # dram__bytes_write.sum, caches flushed before the launch), warp instructions
 # (smsp__inst_executed.sum) and shared-memory wavefronts
 # (l1tex__data_pipe_lsu_wavefronts_mem_shared.sum).  The counts do not depend on
@@ -258,8 +259,8 @@ ALG_BYTES = {
 # fractions of the issue and shared-memory roofs, the ones that bind these
 # kernels (HBM runs at a few percent of peak).
 MEASURED_COUNTERS = {
-    "nfx_spread_sorted": {"radial": {"dram": 17.26e6, "inst": 40.75e6, "smem_wf": 6.39e6},
-                          "clustered": {"dram": 84.82e6, "inst": 78.85e6, "smem_wf": 17.55e6}},
+    "nfx_spread_sorted": {"radial": {"dram": 17.28e6, "inst": 25.26e6, "smem_wf": 4.09e6},
+                          "clustered": {"dram": 85.13e6, "inst": 89.16e6, "smem_wf": 26.74e6}},
     "nfx_interp_sorted": {"radial": {"dram": 13.53e6, "inst": 7.31e6, "smem_wf": 3.71e6},
                           "clustered": {"dram": 102.01e6, "inst": 43.48e6, "smem_wf": 10.11e6}},
 }
@@ -288,7 +289,7 @@ def secondary_roofs(kernel: str, avg_launch_ms: float, sm_mhz) -> dict | None:
         "shared": {"achieved": wf * 128 / t / 1e9, "peak": smem_peak, "unit": "GB/s",
                    "frac": wf * 128 / t / 1e9 / smem_peak, "wavefronts_per_launch": wf},
         "clock_mhz": float(sm_mhz),
-        "counts_from": "ncu --metrics, one launch per point set (profiles/k_spread_interp_2d_counters.md)",
+        "counts_from": "ncu --metrics, one launch per point set (profiles/window_spread.md)",
     }
 
 
