@@ -93,6 +93,12 @@ int nfx_device_status(int* status);
  * bound works. */
 int nfx_selftest_bounded_wait(int* status);
 
+/* Self-test of the kernels' grid-stride walks near the largest M (host only, no
+ * counterpart in the reference): one thread's walk of n positions from `first` in
+ * steps of `stride`, by the function the kernels use.  *visited: positions walked
+ * (at most n / stride + 2), *outside: those not in [0, n). */
+int nfx_selftest_positions(int64_t n, int64_t first, int64_t stride, int64_t* visited, int64_t* outside);
+
 /* Id of the CUDA graph capture the stream takes part in (cudaStreamGetCaptureInfo),
  * 0 when it is not capturing.  Lets a host layer reuse work captured earlier in the
  * same capture (a point sort shared by a type 1 and a type 2). */

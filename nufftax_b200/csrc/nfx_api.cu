@@ -1135,6 +1135,22 @@ int nfx_selftest_bounded_wait(int* status) {
   return nfx_device_status(status);
 }
 
+int nfx_selftest_positions(int64_t n, int64_t first, int64_t stride, int64_t* visited, int64_t* outside) {
+  if (visited == nullptr || outside == nullptr || n < 1 || n > INT32_MAX || first < 0 || first >= n || stride < 1 ||
+      stride > INT32_MAX) {
+    nfx::set_error("nfx_selftest_positions: n, first or stride out of range, or a NULL result");
+    return NFX_ERR_INVALID;
+  }
+  *visited = *outside = 0;
+  const int64_t most = n / stride + 2;
+  int t = (int)first;
+  do {
+    ++*visited;
+    *outside += t < 0 || t >= n;
+  } while (nfx::next_position(t, (unsigned)stride, (int)n) && *visited < most);
+  return NFX_OK;
+}
+
 int nfx_sort_kernel_count(const nfx_opts* opts, int64_t M, int type3, int* n) {
   using namespace nfx;
   if (n == nullptr || M < 0) {

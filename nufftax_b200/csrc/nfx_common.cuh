@@ -90,6 +90,18 @@ __device__ __forceinline__ int wrap_index(int i, int n) {
   return r < 0 ? r + n : r;
 }
 
+// Positions of a sort reach 2^31 - 2, so the position `step` further on may be
+// past int: it is formed and compared as unsigned (step <= 2^31).
+__host__ __device__ __forceinline__ bool position_before(int k, unsigned step, int end) {
+  return (unsigned)k + step < (unsigned)end;
+}
+// Moves k (in [0, end)) `step` positions on; false, and k no position, past the end.
+__host__ __device__ __forceinline__ bool next_position(int& k, unsigned step, int end) {
+  const bool more = position_before(k, step, end);
+  k = (int)((unsigned)k + step);
+  return more;
+}
+
 // ES kernel value phi(z) = exp(beta (sqrt(1 - c z^2) - 1)), zero where the
 // argument is negative (nufftax/core/kernel.py:79-111; arg = 1 - (c z) z).
 template <typename T>

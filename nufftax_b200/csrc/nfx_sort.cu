@@ -602,7 +602,8 @@ __global__ void __launch_bounds__(256) k_sorted_coords(const T* __restrict__ x, 
     __syncthreads();
   }
   const int ngroups = (M + Q - 1) / Q;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < ngroups; t += gridDim.x * blockDim.x) {
+  int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < ngroups) do {
     const int i0 = Q * t;
     int p[Q];
     if (Q % 4 == 0 && i0 + Q - 1 < M) {
@@ -654,7 +655,7 @@ __global__ void __launch_bounds__(256) k_sorted_coords(const T* __restrict__ x, 
         extra[i0 + j] = t3_factor<T>(xr, DIM, g, nq, dz, s_qw);
       }
     }
-  }
+  } while (next_position(t, gridDim.x * blockDim.x, ngroups));
 }
 
 __global__ void k_keys_to_bins(const int* __restrict__ K, int64_t M, int cbits, int* __restrict__ out) {

@@ -327,3 +327,16 @@ def test_sort_kernel_count():
     o3 = make_opts(_lib.NFX_F32, (320, 320, 320), kp, True)
     assert sort_launches(o3, 10_000) == 11
     assert sort_launches(o2, 0) == 2
+
+
+@pytest.mark.parametrize("n", [1, 5000, 2**31 - 303_105, 2**31 - 2])
+def test_grid_stride_walk_ends_at_the_largest_m(n):
+    """The kernels' walk of n positions (n up to the largest accepted M) by 148 * 8
+    CTAs of 256 threads: every thread visits its own positions, all inside [0, n),
+    and stops, although a step past n may leave the int range."""
+    lib = _lib.load()
+    stride = 148 * 8 * 256
+    for first in {0, (n - 1) // 2 % stride, (n - 1) % stride, min(n, stride) - 1}:
+        visited, outside = ctypes.c_int64(), ctypes.c_int64()
+        assert lib.nfx_selftest_positions(n, first, stride, ctypes.byref(visited), ctypes.byref(outside)) == 0
+        assert (visited.value, outside.value) == ((n - 1 - first) // stride + 1, 0)
