@@ -472,6 +472,10 @@ __global__ void k_bin_bounds(const int* __restrict__ Ks, int M, int cbits, int n
 // threads fill the tables together, each locating its subproblem's bin by
 // binary search; otherwise each thread fills its own bins.
 constexpr int kSubSmemBins = 12288;
+// Subproblems of a bin of n points (none for the negative n of corrupt bounds).
+__device__ __forceinline__ int subproblems_of(int n, int maxsub) {
+  return n > 0 ? (int)(((unsigned)n + maxsub - 1) / (unsigned)maxsub) : 0;
+}
 __global__ void k_subproblems(const int* __restrict__ bin_start, int nbins, int maxsub, int max_subs,
                               int* __restrict__ sub_bin, int* __restrict__ sub_start, int* __restrict__ nsub_out) {
   __shared__ int s_warp[32];
@@ -482,7 +486,7 @@ __global__ void k_subproblems(const int* __restrict__ bin_start, int nbins, int 
   const int b0 = min(tid * per, nbins);
   const int b1 = min(b0 + per, nbins);
   int local = 0;
-  for (int b = b0; b < b1; ++b) local += max(bin_start[b + 1] - bin_start[b] + maxsub - 1, 0) / maxsub;
+  for (int b = b0; b < b1; ++b) local += subproblems_of(bin_start[b + 1] - bin_start[b], maxsub);
   int total;
   int excl = block_exclusive_scan(local, s_warp, total);
   const int nsub = min(total, max_subs);  // the tables hold max_subs entries (more only for corrupt bounds)
@@ -490,7 +494,7 @@ __global__ void k_subproblems(const int* __restrict__ bin_start, int nbins, int 
   if (nbins <= kSubSmemBins) {
     for (int b = b0; b < b1; ++b) {
       s_first[b] = excl;
-      excl += max(bin_start[b + 1] - bin_start[b] + maxsub - 1, 0) / maxsub;
+      excl += subproblems_of(bin_start[b + 1] - bin_start[b], maxsub);
     }
     if (tid == 0) s_first[nbins] = total;
     __syncthreads();
@@ -509,7 +513,7 @@ __global__ void k_subproblems(const int* __restrict__ bin_start, int nbins, int 
   } else {
     for (int b = b0; b < b1; ++b) {
       const int e = bin_start[b + 1];
-      for (int q = bin_start[b]; q < e && excl < max_subs; q += maxsub) {
+      for (unsigned q = bin_start[b]; q < (unsigned)e && excl < max_subs; q += maxsub) {
         sub_bin[excl] = b;
         sub_start[excl] = q;
         ++excl;
@@ -601,7 +605,7 @@ __global__ void __launch_bounds__(256) k_sorted_coords(const T* __restrict__ x, 
     }
     __syncthreads();
   }
-  const int ngroups = (M + Q - 1) / Q;
+  const int ngroups = M / Q + (M % Q != 0);
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < ngroups) do {
     const int i0 = Q * t;

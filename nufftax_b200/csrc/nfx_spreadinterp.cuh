@@ -118,6 +118,11 @@ __device__ __forceinline__ void axis_weights(const PointArgs<T>& a, int i0, T xs
   for (int q = 0; q < NS; ++q) w[q] = es_weight(rn_sub((T)(i0 + q), xs), a.beta, a.kc);
 }
 
+// End of the subproblem of bin b that starts at sorted position k0.
+__device__ __forceinline__ int sub_end(const SortView& s, int b, int k0) {
+  return k0 + min(s.maxsub, s.bin_start[b + 1] - k0);
+}
+
 __device__ __forceinline__ void bin_origin(const Geom& g, int b, int& o0, int& o1, int& o2) {
   int bx = b % g.nb[0];
   int r = b / g.nb[0];
@@ -267,19 +272,19 @@ __device__ __forceinline__ void spread_subproblem_cells(const PointArgs<T>& a, c
   const int plane = g.pitch * g.pad[1];
   const int b = a.s.sub_bin[sidx];
   const int k0 = a.s.sub_start[sidx];
-  const int k1 = min(k0 + a.s.maxsub, a.s.bin_start[b + 1]);
+  const int k1 = sub_end(a.s, b, k0);
   int o[3];
   bin_origin(g, b, o[0], o[1], o[2]);
   for (int t = 0; t < a.n_trans; ++t) {
     for (int i = threadIdx.x; i < 2 * tile_cells; i += blockDim.x) s_re[i] = (T)0;
     __syncthreads();
     const int per = ((k1 - k0 + NW - 1) / NW + 31) / 32 * 32;
-    const int w0 = min(k0 + warp * per, k1);
-    const int w1 = min(w0 + per, k1);
-    for (int kb = w0; kb < w1; kb += 32) {
+    const int w0 = k0 + min(warp * per, k1 - k0);
+    const int w1 = w0 + min(per, k1 - w0);
+    for (int kb = w0; (unsigned)kb < (unsigned)w1; kb += 32) {
       const int k = kb + lane;
       const int slot = warp * 32 + lane;
-      if (k < w1) {
+      if ((unsigned)k < (unsigned)w1) {
         const int p = a.s.perm[k];
         int off;
         T w[DIM][NS];
@@ -468,7 +473,7 @@ __device__ __forceinline__ void spread_subproblem_owner(const PointArgs<T>& a, c
   const int plane = g.pitch * g.pad[1];
   const int b = a.s.sub_bin[sidx];
   const int k0 = a.s.sub_start[sidx];
-  const int k1 = min(k0 + a.s.maxsub, a.s.bin_start[b + 1]);
+  const int k1 = sub_end(a.s, b, k0);
   int o[3];
   bin_origin(g, b, o[0], o[1], o[2]);
   const int kx = lane % NS;
@@ -476,9 +481,9 @@ __device__ __forceinline__ void spread_subproblem_owner(const PointArgs<T>& a, c
   const bool lane_on = ky0 < LPR;
   for (int t = 0; t < a.n_trans; ++t) {
     for (int i = threadIdx.x; i < tile_cells; i += blockDim.x) s_tile[i] = CT{(T)0, (T)0};
-    for (int kb = k0; kb < k1; kb += NT) {
-      const int k = kb + threadIdx.x;
-      if (k < k1) {
+    for (unsigned kb = k0; kb < (unsigned)k1; kb += NT) {
+      const unsigned k = kb + threadIdx.x;
+      if (k < (unsigned)k1) {
         const int p = a.s.perm[k];
         T xv[3];
         load_sorted<T, 3>(a, k, xv);
@@ -525,7 +530,7 @@ __device__ __forceinline__ void spread_subproblem_owner(const PointArgs<T>& a, c
         }
       }
       __syncthreads();  // also orders the tile zeroing before the first adds
-      const int cnt = min(NT, k1 - kb);
+      const int cnt = min(NT, k1 - (int)kb);
       static_assert((NW & (NW - 1)) == 0, "warps per CTA a power of two");
       // planes of each footprint this warp owns: dz0 + pl * NW < NS, at most
       // ceil(NS / NW) (exactly NS / NW when NW divides NS)
@@ -771,14 +776,14 @@ struct WarpPoints {
 
 __device__ __forceinline__ int round_perm(const SortView& s, int kb, int k1) {
   const int k = kb + (threadIdx.x & 31);
-  return k < k1 ? s.perm[k] : -1;
+  return (unsigned)k < (unsigned)k1 ? s.perm[k] : -1;  // kb may be past the last position (and int)
 }
 
 template <typename T, int DIM>
 __device__ __forceinline__ void round_coords(const PointArgs<T>& a, int kb, int k1, T (&xv)[3]) {
   const int k = kb + (threadIdx.x & 31);
 #pragma unroll
-  for (int d = 0; d < 3; ++d) xv[d] = (d < DIM && k < k1) ? sorted_coord(a, d, k) : (T)0;
+  for (int d = 0; d < 3; ++d) xv[d] = (d < DIM && (unsigned)k < (unsigned)k1) ? sorted_coord(a, d, k) : (T)0;
 }
 
 template <typename T, int DIM, int NS>
@@ -842,7 +847,7 @@ __device__ __forceinline__ void interp_group(const PointArgs<T>& a, const cplx_t
   }
   const int b = a.s.sub_bin[sidx];
   const int k0 = a.s.sub_start[sidx];
-  const int k1 = min(k0 + a.s.maxsub, a.s.bin_start[b + 1]);
+  const int k1 = sub_end(a.s, b, k0);
   int o[3];
   bin_origin(g, b, o[0], o[1], o[2]);
   for (int t = 0; t < a.n_trans; ++t) {
@@ -853,7 +858,7 @@ __device__ __forceinline__ void interp_group(const PointArgs<T>& a, const cplx_t
     int p_cur = round_perm(a.s, k0 + warp * 32, k1);
     T x_cur[3];
     round_coords<T, DIM>(a, k0 + warp * 32, k1, x_cur);
-    for (int kb = k0 + warp * 32; kb < k1; kb += kStep) {  // warp-uniform
+    for (unsigned kb = k0 + warp * 32; kb < (unsigned)k1; kb += kStep) {  // warp-uniform
       const int p_next = round_perm(a.s, kb + kStep, k1);
       T x_next[3];
       round_coords<T, DIM>(a, kb + kStep, k1, x_next);
@@ -861,7 +866,7 @@ __device__ __forceinline__ void interp_group(const PointArgs<T>& a, const cplx_t
       p_cur = p_next;
 #pragma unroll
       for (int d = 0; d < 3; ++d) x_cur[d] = x_next[d];
-      const int npts = min(32, k1 - kb);
+      const int npts = min(32, k1 - (int)kb);
       for (int j0 = 0; j0 < npts; j0 += PPW) {
         const int j = j0 + lane / GL;
         const bool valid = j < npts;
@@ -954,7 +959,7 @@ __device__ __forceinline__ void interp_subproblem(const PointArgs<T>& a, const c
   {
     const int b = a.s.sub_bin[sidx];
     const int k0 = a.s.sub_start[sidx];
-    const int k1 = min(k0 + a.s.maxsub, a.s.bin_start[b + 1]);
+    const int k1 = sub_end(a.s, b, k0);
     int o[3];
     bin_origin(g, b, o[0], o[1], o[2]);
     for (int t = 0; t < a.n_trans; ++t) {
@@ -965,17 +970,17 @@ __device__ __forceinline__ void interp_subproblem(const PointArgs<T>& a, const c
       // entry and folded coordinates (both in sorted order)
       const int kStep = blockDim.x;
       int k = k0 + threadIdx.x;
-      int p_cur = k < k1 ? a.s.perm[k] : 0;
+      int p_cur = (unsigned)k < (unsigned)k1 ? a.s.perm[k] : 0;
       T x_cur[DIM];
 #pragma unroll
-      for (int d = 0; d < DIM; ++d) x_cur[d] = k < k1 ? sorted_coord(a, d, k) : (T)0;
-      for (; k < k1; k += kStep) {
+      for (int d = 0; d < DIM; ++d) x_cur[d] = (unsigned)k < (unsigned)k1 ? sorted_coord(a, d, k) : (T)0;
+      for (; (unsigned)k < (unsigned)k1; k += kStep) {
         const int p = p_cur;
         T xv[DIM];
 #pragma unroll
         for (int d = 0; d < DIM; ++d) xv[d] = x_cur[d];
         {
-          const bool more = k + kStep < k1;
+          const bool more = position_before(k, kStep, k1);
           p_cur = more ? a.s.perm[k + kStep] : 0;
 #pragma unroll
           for (int d = 0; d < DIM; ++d) x_cur[d] = more ? sorted_coord(a, d, k + kStep) : (T)0;
@@ -1134,7 +1139,7 @@ __device__ __forceinline__ bool grad_group(const PointArgs<T>& a, const cplx_t<T
   T* dout = kx == 1 ? dx : (kx == 2 ? dy : (kx == 3 ? dz : nullptr));
   const int b = a.s.sub_bin[sidx];
   const int k0 = a.s.sub_start[sidx];
-  const int k1 = min(k0 + a.s.maxsub, a.s.bin_start[b + 1]);
+  const int k1 = sub_end(a.s, b, k0);
   int o[3];
   bin_origin(g, b, o[0], o[1], o[2]);
   for (int t = 0; t < a.n_trans; ++t) {
@@ -1150,14 +1155,14 @@ __device__ __forceinline__ bool grad_group(const PointArgs<T>& a, const cplx_t<T
     CT v_cur;
     v_cur.x = v_cur.y = (T)0;
     if (p_cur >= 0) v_cur = V[(int64_t)t * a.M + p_cur];
-    for (int kb = kw; kb < k1; kb += kStep) {  // warp-uniform
+    for (unsigned kb = kw; kb < (unsigned)k1; kb += kStep) {  // warp-uniform
       const WarpPoints<T> wp = warp_points<T, 3, NS>(a, p_cur, x_cur, o, row, plane);
       const CT vv = v_cur;
       p_cur = p_next;
       p_next = round_perm(a.s, kb + 2 * kStep, k1);
       round_coords<T, 3>(a, kb + kStep, k1, x_cur);
       if (p_cur >= 0) v_cur = V[(int64_t)t * a.M + p_cur];
-      const int npts = min(32, k1 - kb);
+      const int npts = min(32, k1 - (int)kb);
 #pragma unroll 1
       for (int j0 = 0; j0 < npts; j0 += PPW) {
         const int j = j0 + lane / GL;
@@ -1231,8 +1236,16 @@ __device__ __forceinline__ bool grad_group(const PointArgs<T>& a, const cplx_t<T
 // ---------------------------------------------------------------------------
 // Gradient pass (see launch_grad in nfx_internal.h)
 // ---------------------------------------------------------------------------
+// CTAs per SM the gradient pass's registers must allow for (0: the compiler's
+// choice).  1D complex128 at small widths runs on its residency: ns 6, 2M points,
+// 107 us with four CTAs, 116 with three.
+template <typename T, int DIM, int NS>
+constexpr int grad_min_ctas() {
+  return sizeof(T) == 8 && DIM == 1 && NS <= 6 ? (NS == 2 ? 5 : 4) : 0;
+}
+
 template <typename T, int DIM, int NS, int NW>
-__global__ void __launch_bounds__(NW * 32) k_grad(const __grid_constant__ PointArgs<T> a, const cplx_t<T>* __restrict__ G,
+__global__ void __launch_bounds__(NW * 32, grad_min_ctas<T, DIM, NS>()) k_grad(const __grid_constant__ PointArgs<T> a, const cplx_t<T>* __restrict__ G,
                                                   const cplx_t<T>* __restrict__ V, cplx_t<T>* __restrict__ out_interp,
                                                   T* __restrict__ dx, T* __restrict__ dy, T* __restrict__ dz,
                                                   const __grid_constant__ CUtensorMap tmap) {
@@ -1263,7 +1276,7 @@ __global__ void __launch_bounds__(NW * 32) k_grad(const __grid_constant__ PointA
       }
     }
     const int k0 = a.s.sub_start[sidx];
-    const int k1 = min(k0 + a.s.maxsub, a.s.bin_start[b + 1]);
+    const int k1 = sub_end(a.s, b, k0);
     int o[3];
     bin_origin(g, b, o[0], o[1], o[2]);
     for (int t = 0; t < a.n_trans; ++t) {
@@ -1274,23 +1287,23 @@ __global__ void __launch_bounds__(NW * 32) k_grad(const __grid_constant__ PointA
       // ahead, folded coordinates (sorted order) and V one iteration ahead
       const int kStep = blockDim.x;
       int k = k0 + threadIdx.x;
-      int p_cur = k < k1 ? a.s.perm[k] : 0;
-      int p_next = k + kStep < k1 ? a.s.perm[k + kStep] : 0;
+      int p_cur = (unsigned)k < (unsigned)k1 ? a.s.perm[k] : 0;
+      int p_next = position_before(k, kStep, k1) ? a.s.perm[k + kStep] : 0;
       T x_cur[DIM];
       CT v_cur;
       v_cur.x = v_cur.y = (T)0;
 #pragma unroll
-      for (int d = 0; d < DIM; ++d) x_cur[d] = k < k1 ? sorted_coord(a, d, k) : (T)0;
-      if (k < k1) v_cur = V[(int64_t)t * a.M + p_cur];
-      for (; k < k1; k += kStep) {
+      for (int d = 0; d < DIM; ++d) x_cur[d] = (unsigned)k < (unsigned)k1 ? sorted_coord(a, d, k) : (T)0;
+      if ((unsigned)k < (unsigned)k1) v_cur = V[(int64_t)t * a.M + p_cur];
+      for (; (unsigned)k < (unsigned)k1; k += kStep) {
         const int p = p_cur;
         T xv[DIM];
 #pragma unroll
         for (int d = 0; d < DIM; ++d) xv[d] = x_cur[d];
         const CT vv = v_cur;
         {
-          const bool more = k + kStep < k1;
-          const int p_after = k + 2 * kStep < k1 ? a.s.perm[k + 2 * kStep] : 0;
+          const bool more = position_before(k, kStep, k1);
+          const int p_after = position_before(k, 2 * kStep, k1) ? a.s.perm[k + 2 * kStep] : 0;
 #pragma unroll
           for (int d = 0; d < DIM; ++d) x_cur[d] = more ? sorted_coord(a, d, k + kStep) : (T)0;
           if (more) v_cur = V[(int64_t)t * a.M + p_next];

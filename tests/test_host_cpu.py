@@ -336,7 +336,9 @@ def test_grid_stride_walk_ends_at_the_largest_m(n):
     and stops, although a step past n may leave the int range."""
     lib = _lib.load()
     stride = 148 * 8 * 256
-    for first in {0, (n - 1) // 2 % stride, (n - 1) % stride, min(n, stride) - 1}:
+    last = (n - 1) // stride * stride  # a subproblem's rounds (256 points) start anywhere up to n - 1
+    for first, stride in [(f, stride) for f in {0, (n - 1) // 2 % stride, (n - 1) % stride, min(n, stride) - 1}] + [
+            (f, s) for f in (last, n - 1) for s in (256, 512)]:
         visited, outside = ctypes.c_int64(), ctypes.c_int64()
         assert lib.nfx_selftest_positions(n, first, stride, ctypes.byref(visited), ctypes.byref(outside)) == 0
         assert (visited.value, outside.value) == ((n - 1 - first) // stride + 1, 0)
