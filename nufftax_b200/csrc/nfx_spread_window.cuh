@@ -118,21 +118,35 @@ size_t win_smem_bytes() {
          (WinShape<T, DIM, NS>::GROUP ? kWinBlocks * sizeof(int) + kWinRound * sizeof(unsigned short) : 0);
 }
 
-// Points of one work item of a spread of M points on `ctas` resident CTAs: the
-// items are equal, so as many as the CTAs take in whole rounds, of at most
+// Work items of a spread of M points on `ctas` resident CTAs: points of one item,
+// and the items of a group that one CTA takes when their points share a block.
+// The items are equal, so as many as the CTAs take in whole rounds, of at most
 // kWinRound points (2D: 1024; 4M clustered points 146 us, 159 with 2048, whose
 // four rounds end unevenly).  The least size bounds the partial sums a crowded
-// cell gets (each slice of a warp adds its own, and their float rounding): 100 k
-// points in one 2D cell have a relative error of 2.5e-6 with 64-point items,
-// 1.5e-6 with 256, 0.9e-6 with 512 and no less with more.  3D points cost several
-// times a 2D point and spread over more cells, so their items may be smaller;
-// sets too small to give every SM an item of the least size are cut down to 64.
-inline int win_part_points(int dim, int64_t M, int ctas) {
+// cell gets (each slice of a warp adds its own, and their float rounding).  3D
+// points cost several times a 2D point and spread over more cells, so their items
+// may be smaller; sets too small to give every SM an item of the least size are
+// cut down to 64.
+// Groups (2D) reach the size of a subproblem, so that a crowded cell gets no more
+// partial sums than one tile per subproblem would send.  Float error of 2D points in
+// one cell, over the root of the sum of squares: 100 k 2.0e-7, 1M 4.2e-7, 4M 5.6e-7
+// (by shared-memory tiles 2.9e-7, 5.9e-7, 7.4e-7; every slice by itself 5.9e-7,
+// 1.2e-6, 2.2e-6); 1M 3D points 5.9e-7 (4.7e-7, 9.7e-7).
+// Spreads of at most 512 slices send every slice by itself (group 0).  8M points in
+// few blocks, ns 6: 341 us, 286 without groups, 314 by shared-memory tiles.
+struct WinSplit {
+  int part, group;
+};
+inline WinSplit win_split(int dim, int warps, int64_t M, int ctas, int maxsub) {
   const int64_t most = dim == 2 ? 1024 : kWinRound;
   const int64_t least = M < 256 * 148 ? 64 : (dim == 2 ? 512 : 128);
   const int64_t rounds = (M + ctas * most - 1) / (ctas * most);
-  const int64_t n = rounds > 0 ? (M + ctas * rounds - 1) / (ctas * rounds) : 1;
-  return (int)((n < least ? least : n) + 31) / 32 * 32;
+  int group = dim == 2 ? (int)(maxsub < most ? 1 : (maxsub > 4 * most ? 4 : maxsub / most)) : 1;
+  int64_t n = rounds > 0 ? (M + ctas * rounds - 1) / (ctas * rounds) : 1;
+  n = ((n < least ? least : n) + 31) / 32 * 32;
+  if (dim == 2 && rounds <= 1 && maxsub > n) group = (int)(maxsub / n < 16 ? maxsub / n : 16);
+  if (M * warps <= 512 * n) group = 0;
+  return WinSplit{(int)n, group};
 }
 
 // Adds one point whose strength or coordinates are not finite cell by cell
@@ -222,6 +236,13 @@ struct Window<T, 2, NS> {
   using CT = cplx_t<T>;
   using PT = typename PairOf<T>::type;
   using W = WinShape<T, 2, NS>;
+  static constexpr int CELLS = W::RL;
+  // Grid index of a lane's cell i of the window that starts at `first`; -1: none.
+  static __device__ __forceinline__ int cell_at(const Geom& g, int i, int lane, const int (&first)[3]) {
+    const int x = lane % W::LW, row = (lane / W::LW) * W::RL + i;
+    if (first[0] < 0 || x >= W::WX || row >= W::WY) return -1;
+    return wrap_mod(first[1] + row, 1, g) * g.nf[0] + wrap_mod(first[0] + x, 0, g);
+  }
   PT acc[W::RL];  // complex cells of this lane's rows
   int xo, yo;     // this lane's entries of a slot
 
@@ -230,6 +251,7 @@ struct Window<T, 2, NS> {
     yo = W::YO + (lane / W::LW) * W::RS;
     clear();
   }
+  __device__ __forceinline__ PT& cell(int i) { return acc[i]; }
   __device__ __forceinline__ void clear() {
 #pragma unroll
     for (int i = 0; i < W::RL; ++i) acc[i] = pair_of((T)0, (T)0);
@@ -249,9 +271,35 @@ struct Window<T, 2, NS> {
       }
     }
   }
-  __device__ __forceinline__ void add(const T* sp) {
+  __device__ __forceinline__ void add(const T* sp) { add_to(acc, sp); }
+  __device__ __forceinline__ void add_to(PT (&sum)[W::RL], const T* sp) {
     const PT cw = *reinterpret_cast<const PT*>(sp + xo);
-    for_weights<W::RL>(sp + yo, [&](int r, T w) { acc[r] = fma2(pair_of(w, w), cw, acc[r]); });
+    for_weights<W::RL>(sp + yo, [&](int r, T w) { sum[r] = fma2(pair_of(w, w), cw, sum[r]); });
+  }
+  // Points j .. je - 1 of one block, four at a time.  A crowded block's alternate
+  // between two sums, which halves the length (and float rounding) of each.
+  __device__ __forceinline__ void add_run(const T*& sp, int& j, int je, bool crowded) {
+    if (sizeof(T) == 4 && crowded) {
+      PT other[W::RL];
+#pragma unroll
+      for (int r = 0; r < W::RL; ++r) other[r] = pair_of((T)0, (T)0);
+      for (; j + 4 <= je; j += 4, sp += 4 * W::SLOT) {
+#pragma unroll
+        for (int q = 0; q < 4; q += 2) {
+          add(sp + q * W::SLOT);
+          add_to(other, sp + (q + 1) * W::SLOT);
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < W::RL; ++r) acc[r] = add2(acc[r], other[r]);
+    } else {
+      for (; j + 4 <= je; j += 4, sp += 4 * W::SLOT) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) add(sp + q * W::SLOT);
+      }
+    }
+#pragma unroll 1
+    for (; j < je; ++j, sp += W::SLOT) add(sp);
   }
   // (ox, oy, oz): the window's first cell per axis (inside the grid)
   __device__ __forceinline__ void flush(const Geom& g, int ox, int oy, int, int lane, CT* __restrict__ out) {
@@ -280,6 +328,14 @@ struct Window<T, 3, NS> {
   using CT = cplx_t<T>;
   using PT = typename PairOf<T>::type;
   using W = WinShape<T, 3, NS>;
+  static constexpr int CELLS = W::NCOL * W::WZ;
+  // As in 2D.
+  static __device__ __forceinline__ int cell_at(const Geom& g, int i, int lane, const int (&first)[3]) {
+    const int c = lane + 32 * (i / W::WZ);
+    if (first[0] < 0 || c >= W::NC) return -1;
+    return (wrap_mod(first[2] + i % W::WZ, 2, g) * g.nf[1] + wrap_mod(first[1] + c / W::WX, 1, g)) * g.nf[0] +
+           wrap_mod(first[0] + c % W::WX, 0, g);
+  }
   PT acc[W::NCOL][W::WZ];      // complex cells
   int xo[W::NCOL], yo[W::NCOL];  // this lane's columns' entries of a slot
 
@@ -292,6 +348,7 @@ struct Window<T, 3, NS> {
     }
     clear();
   }
+  __device__ __forceinline__ PT& cell(int i) { return acc[i / W::WZ][i % W::WZ]; }
   __device__ __forceinline__ void clear() {
 #pragma unroll
     for (int i = 0; i < W::NCOL; ++i)
@@ -322,6 +379,14 @@ struct Window<T, 3, NS> {
       for (int i = 0; i < W::NCOL; ++i) acc[i][k] = fma2(zd, v[i], acc[i][k]);
     });
   }
+  __device__ __forceinline__ void add_run(const T*& sp, int& j, int je, bool) {
+    for (; j + 2 <= je; j += 2, sp += 2 * W::SLOT) {
+      add(sp);
+      add(sp + W::SLOT);
+    }
+#pragma unroll 1
+    for (; j < je; ++j, sp += W::SLOT) add(sp);
+  }
   __device__ __forceinline__ void flush(const Geom& g, int ox, int oy, int oz, int lane, CT* __restrict__ out) {
     const int plane = g.nf[0] * g.nf[1];  // grids have fewer than 2^31 cells
     int at[W::NCOL];
@@ -350,23 +415,117 @@ struct Window<T, 3, NS> {
   }
 };
 
-// One work item: `a.win_part` consecutive points of the sorted order (of one
-// or several bins).  The CTA groups them by block, then every warp takes a
-// contiguous slice of the grouped list 32 points at a time: each lane stages
-// one point, and the warp adds the 32 one after another, flushing the window
-// whenever the block changes.  The next 32 points are fetched while the
+// Block of a point's cell within its tile, from its composite key.
+template <typename T, int DIM, int NS>
+__device__ __forceinline__ int key_block(const Geom& g, int cell) {
+  using W = WinShape<T, DIM, NS>;
+  const int nbx = (g.tile[0] + W::BX - 1) / W::BX, nby = (g.tile[1] + W::BY - 1) / W::BY;
+  const int r = fast_div(cell, g.tdiv[0]);
+  const int cx = cell - r * g.tile[0];
+  if (DIM == 2) return r / W::BY * nbx + cx / W::BX;
+  const int cz = fast_div(r, g.tdiv[1]);
+  const int cy = r - cz * g.tile[1];
+  return (cz / W::BZ * nby + cy / W::BY) * nbx + cx / W::BX;
+}
+template <typename T, int DIM, int NS>
+__device__ __forceinline__ bool same_block(const PointArgs<T>& a, int key, int other) {
+  const int cmask = (1 << a.s.cbits) - 1;
+  return key >> a.s.cbits == other >> a.s.cbits &&
+         key_block<T, DIM, NS>(a.g, key & cmask) == key_block<T, DIM, NS>(a.g, other & cmask);
+}
+
+// Sends the open windows of a crowded item's warps (whose points share a block) to
+// the grid as their sum, formed in the slots' shared memory by all warps.  Every
+// addition to a grid cell rounds at the size of the whole sum: what a crowded block
+// sends should be few large partial sums.  Returns whether this warp still holds a
+// window: one of another block than the first warp's (tiles that are no multiple of
+// the block) stays with its warp.
+template <typename T, int DIM, int NS, int NW>
+__device__ __forceinline__ bool send_sum(Window<T, DIM, NS>& win, const int (&cur)[3], const Geom& g, T* s_slots,
+                                         int warp, int lane, cplx_t<T>* __restrict__ out) {
+  using PT = typename PairOf<T>::type;
+  using W = WinShape<T, DIM, NS>;
+  constexpr int CELLS = Window<T, DIM, NS>::CELLS;
+  constexpr int PER = W::SLOT / 2;  // cells a lane that a warp's slots hold
+  __shared__ int s_cur[NW][3];
+  PT* const buf = reinterpret_cast<PT*>(s_slots) + lane;  // warp w's cells start at w * 32 * PER
+  if (lane < 3) s_cur[warp][lane] = lane == 0 ? cur[0] : (lane == 1 ? cur[1] : cur[2]);
+  auto same = [&](int w) {
+    return s_cur[w][0] == s_cur[0][0] && s_cur[w][1] == s_cur[0][1] && s_cur[w][2] == s_cur[0][2];
+  };
+#pragma unroll
+  for (int h = 0; h < CELLS; h += PER) {
+    __syncthreads();  // the slots' points, or the cells of the part before, are done with
+#pragma unroll
+    for (int i = h; i < CELLS && i < h + PER; ++i) buf[(warp * PER + i - h) * 32] = win.cell(i);
+    __syncthreads();
+#pragma unroll 1
+    for (int i = h + warp; i < CELLS && i < h + PER; i += NW) {
+      const int at = Window<T, DIM, NS>::cell_at(g, i, lane, s_cur[0]);
+      if (at < 0) continue;
+      PT sum = buf[(i - h) * 32];
+#pragma unroll 1
+      for (int w = 1; w < NW; ++w)
+        if (same(w)) sum = add2(sum, buf[(w * PER + i - h) * 32]);
+      red_add(out + at, unpair(sum));
+    }
+  }
+  const bool sent = same(warp);
+  __syncthreads();
+  if (sent) win.clear();
+  return !sent && cur[0] >= 0;
+}
+
+// First point and points of the group of items that `item` belongs to.
+template <typename T>
+__device__ __forceinline__ int win_group_points(const PointArgs<T>& a, int item, int& n) {
+  const int k = (item - item % a.win_group) * a.win_part;
+  n = (int)min((int64_t)a.win_part * a.win_group, a.M - k);
+  return k;
+}
+// The keys of that group's first and last point, in lanes 0 and 1.  An ungrouped
+// kernel loads them an item ahead; grouping waits for keys anyway.
+template <typename T>
+__device__ __forceinline__ int win_group_keys(const PointArgs<T>& a, int item) {
+  if (a.win_group == 0) return 0;
+  int n;
+  const int k = win_group_points(a, item, n), lane = threadIdx.x & 31;
+  return lane < 2 ? a.s.keys[lane == 0 ? k : k + n - 1] : 0;
+}
+
+// One work item: `a.win_part` consecutive points of the sorted order (of one or
+// several bins); ahead: its win_group_keys (ungrouped).  The CTA groups them by block,
+// then every warp takes a contiguous slice of the grouped list 32 points at a time:
+// each lane stages one point, and the warp adds the 32 one after another, flushing
+// the window whenever the block changes.  The next 32 points are fetched while the
 // current ones are added.
+// A crowded item: when all points of a group of `a.win_group` items lie in one
+// block, one of them takes the whole group and the others nothing, and its warps
+// send one window.  Which one rotates with the group's place in the grid-stride
+// order, so that each CTA gets its share.
 template <typename T, int DIM, int NS, int NW>
 __device__ __forceinline__ void spread_window(const PointArgs<T>& a, const cplx_t<T>* __restrict__ c,
-                                              cplx_t<T>* __restrict__ fw, int item, unsigned char* smem_raw) {
+                                              cplx_t<T>* __restrict__ fw, int item, int ahead,
+                                              unsigned char* smem_raw) {
   using CT = cplx_t<T>;
   using W = WinShape<T, DIM, NS>;
   constexpr int NT = NW * 32;
   constexpr int PER = (kWinRound + NT - 1) / NT;  // most points of an item per thread
   __shared__ int s_warp[32];
   const Geom& g = a.g;
-  const int k0 = item * a.win_part;
-  const int n = (int)min((int64_t)a.win_part, a.M - k0);
+  int k0 = item * a.win_part;
+  int n = (int)min((int64_t)a.win_part, a.M - k0);
+  const int first_key = W::GROUP ? a.s.keys[k0] : 0, last_key = W::GROUP ? a.s.keys[k0 + n - 1] : 0;
+  const int ends = W::GROUP && DIM == 2 ? win_group_keys(a, item) : ahead;
+  const bool one_block =
+      a.win_group > 0 && (DIM == 3 ? same_block<T, DIM, NS>(a, first_key, last_key)  // groups of one
+                                   : same_block<T, DIM, NS>(a, __shfl_sync(0xffffffffu, ends, 0),
+                                                            __shfl_sync(0xffffffffu, ends, 1)));
+  if (one_block) {
+    k0 = win_group_points(a, item, n);
+    const unsigned members = (unsigned)((n + a.win_part - 1) / a.win_part);
+    if (item % a.win_group != (int)((unsigned)item / gridDim.x % members)) return;
+  }
   T* s_slots = reinterpret_cast<T*>(smem_raw);
   int* s_cnt = reinterpret_cast<int*>(s_slots + NT * W::SLOT);  // per block: points, then its list start
   unsigned short* s_list = reinterpret_cast<unsigned short*>(s_cnt + kWinBlocks);
@@ -374,15 +533,14 @@ __device__ __forceinline__ void spread_window(const PointArgs<T>& a, const cplx_
   T* my_slot = s_slots + (warp * 32 + lane) * W::SLOT;
   const T* warp_slots = s_slots + warp * 32 * W::SLOT;
   // ---- group the points by block: bins in order, blocks within a bin ----
+  bool listed = false;
   if constexpr (W::GROUP) {
-    const int nbx = (g.tile[0] + W::BX - 1) / W::BX, nby = (g.tile[1] + W::BY - 1) / W::BY;
-    const int nbz = (g.tile[2] + W::BZ - 1) / W::BZ;
-    const int bin0 = a.s.keys[k0] >> a.s.cbits;
-    const int64_t span = (int64_t)((a.s.keys[k0 + n - 1] >> a.s.cbits) - bin0 + 1) * (nbx * nby * nbz);
-    if (span > kWinBlocks || span < 1) {
-      // few points per bin: no two of them are likely to share a block
-      for (int i = threadIdx.x; i < n; i += NT) s_list[i] = (unsigned short)i;
-    } else {
+    const int per_bin = key_block<T, DIM, NS>(g, g.tile[0] * g.tile[1] * g.tile[2] - 1) + 1;  // blocks
+    const int bin0 = first_key >> a.s.cbits;
+    const int64_t span = (int64_t)((last_key >> a.s.cbits) - bin0 + 1) * per_bin;
+    // more: few points per bin, no two of them are likely to share a block
+    listed = !one_block && span <= kWinBlocks && span >= 1;
+    if (listed) {
       const int nblk = (int)span;
       const int cmask = (1 << a.s.cbits) - 1;
       for (int i = threadIdx.x; i < nblk; i += NT) s_cnt[i] = 0;
@@ -396,17 +554,7 @@ __device__ __forceinline__ void spread_window(const PointArgs<T>& a, const cplx_
 #pragma unroll
       for (int i = 0; i < PER; ++i) {
         if (key[i] >= 0) {
-          const int cell = key[i] & cmask;
-          const int r = fast_div(cell, g.tdiv[0]);
-          const int cx = cell - r * g.tile[0];
-          int blk = (key[i] >> a.s.cbits) - bin0;
-          if (DIM == 2) {
-            blk = (blk * nby + r / W::BY) * nbx + cx / W::BX;
-          } else {
-            const int cz = fast_div(r, g.tdiv[1]);
-            const int cy = r - cz * g.tile[1];
-            blk = ((blk * nbz + cz / W::BZ) * nby + cy / W::BY) * nbx + cx / W::BX;
-          }
+          const int blk = ((key[i] >> a.s.cbits) - bin0) * per_bin + key_block<T, DIM, NS>(g, key[i] & cmask);
           key[i] = min(max(blk, 0), nblk - 1);  // keys of a sound sort are in range
           rank[i] = atomicAdd(&s_cnt[key[i]], 1);
         }
@@ -426,113 +574,106 @@ __device__ __forceinline__ void spread_window(const PointArgs<T>& a, const cplx_
 #pragma unroll
       for (int i = 0; i < PER; ++i)
         if (key[i] >= 0) s_list[s_cnt[key[i]] + rank[i]] = (unsigned short)(i * NT + threadIdx.x);
+      __syncthreads();
     }
-    __syncthreads();
   }
   // ---- the warp's slice of the list, per transform ----
-  auto list_at = [&](int i) { return W::GROUP ? (int)s_list[i] : i; };
-  const int p0 = (int)((unsigned)n * warp / NW);  // slices differ by at most one point
-  const int p1 = (int)((unsigned)n * (warp + 1) / NW);
-  if (p0 < p1) {
-    Window<T, DIM, NS> win(lane);
-    for (int t = 0; t < a.n_trans; ++t) {
-      const CT* ct = c + (int64_t)t * a.M;
-      CT* const out = fw + (int64_t)t * a.grid_stride;
-      // this lane's point of the next 32 (kn < 0: none), two list entries ahead
-      T xn[DIM];
-      CT cn;
-      zero_pair<T>(cn);
+  auto list_at = [&](int i) { return W::GROUP && listed ? (int)s_list[i] : i; };
+  const int p0 = (int)((int64_t)n * warp / NW);  // slices differ by at most one point
+  const int p1 = (int)((int64_t)n * (warp + 1) / NW);
+  Window<T, DIM, NS> win(lane);
+  for (int t = 0; t < a.n_trans; ++t) {
+    const CT* ct = c + (int64_t)t * a.M;
+    CT* const out = fw + (int64_t)t * a.grid_stride;
+    // this lane's point of the next 32 (kn < 0: none), two list entries ahead
+    T xn[DIM];
+    CT cn;
+    zero_pair<T>(cn);
 #pragma unroll
-      for (int d = 0; d < DIM; ++d) xn[d] = (T)0;
-      int kn = p0 + lane < p1 ? k0 + list_at(p0 + lane) : -1;
+    for (int d = 0; d < DIM; ++d) xn[d] = (T)0;
+    int kn = p0 + lane < p1 ? k0 + list_at(p0 + lane) : -1;
+    if (kn >= 0) {
+      load_sorted<T, DIM>(a, kn, xn);
+      cn = ct[a.s.perm[kn]];
+    }
+    int k2 = p0 + 32 + lane < p1 ? k0 + list_at(p0 + 32 + lane) : -1;
+    int pn = k2 >= 0 ? a.s.perm[k2] : 0;
+    int cur[3] = {-1, -1, -1};  // the open window's first cell per axis, -1: none
+    for (int p = p0; p < p1; p += 32) {
+      const int cnt = min(32, p1 - p);
+      const int k = kn;
+      T xv[DIM];
+#pragma unroll
+      for (int d = 0; d < DIM; ++d) xv[d] = xn[d];
+      CT cv = cn;
+      kn = k2;
       if (kn >= 0) {
         load_sorted<T, DIM>(a, kn, xn);
-        cn = ct[a.s.perm[kn]];
+        cn = ct[pn];
       }
-      int k2 = p0 + 32 + lane < p1 ? k0 + list_at(p0 + 32 + lane) : -1;
-      int pn = k2 >= 0 ? a.s.perm[k2] : 0;
-      int cur[3] = {-1, -1, -1};  // the open window's first cell per axis, -1: none
-      for (int p = p0; p < p1 + 32; p += 32) {
-        const int cnt = min(32, p1 - p);  // <= 0 on the last trip, which only flushes
-        const int k = kn;
-        T xv[DIM];
+      k2 = p + 64 + lane < p1 ? k0 + list_at(p + 64 + lane) : -1;
+      pn = k2 >= 0 ? a.s.perm[k2] : 0;
+      // stage this lane's point, axis by axis (points added directly stage zeros)
+      int base[3] = {0, 0, 0};
+      int i0[DIM], dl[DIM];
+      bool fin = true;
 #pragma unroll
-        for (int d = 0; d < DIM; ++d) xv[d] = xn[d];
-        CT cv = cn;
-        kn = k2;
-        if (kn >= 0) {
-          load_sorted<T, DIM>(a, kn, xn);
-          cn = ct[pn];
-        }
-        k2 = p + 64 + lane < p1 ? k0 + list_at(p + 64 + lane) : -1;
-        pn = k2 >= 0 ? a.s.perm[k2] : 0;
-        // stage this lane's point, axis by axis (points added directly stage zeros)
-        int base[3] = {-1, -1, -1};
-        if (cnt > 0) {
-          int i0[DIM], dl[DIM];
-          bool fin = true;
-#pragma unroll
-          for (int d = 0; d < DIM; ++d) {
-            constexpr int kB[3] = {W::BX, W::BY, W::BZ};
-            i0[d] = left_cell<T, NS>(xv[d]);
-            const int l = wrap_index(i0[d], g.nf[d]);
-            base[d] = (int)((unsigned)l / kB[d]) * kB[d];
-            dl[d] = l - base[d];
-            fin = fin && is_finite(xv[d]);
-          }
-          if (k >= 0) cv = with_extra(a, k, cv);
-          fin = fin && is_finite(cv.x) && is_finite(cv.y);
-          if (k >= 0 && !fin) win_add_direct<T, DIM, NS>(a, cv, xv[0], xv[1], xv[DIM - 1], out);
-          if (k < 0 || !fin) {
-            zero_pair<T>(cv);
-#pragma unroll
-            for (int d = 0; d < DIM; ++d) {
-              dl[d] = i0[d] = 0;
-              xv[d] = (T)(NS / 2);
-            }
-          }
-          T w[NS];
-          axis_weights<T, NS>(a, i0[0], xv[0], w);
-          Window<T, DIM, NS>::template stage<0>(my_slot, cv, w, dl[0]);
-          axis_weights<T, NS>(a, i0[1], xv[1], w);
-          Window<T, DIM, NS>::template stage<1>(my_slot, cv, w, dl[1]);
-          if constexpr (DIM == 3) {
-            axis_weights<T, NS>(a, i0[2], xv[2], w);
-            Window<T, DIM, NS>::template stage<2>(my_slot, cv, w, dl[2]);
-          }
-        }
-        // lane j starts a block when its block differs from point j - 1's
-        bool differs = false;
+      for (int d = 0; d < DIM; ++d) {
+        constexpr int kB[3] = {W::BX, W::BY, W::BZ};
+        i0[d] = left_cell<T, NS>(xv[d]);
+        const int l = wrap_index(i0[d], g.nf[d]);
+        base[d] = (int)((unsigned)l / kB[d]) * kB[d];
+        dl[d] = l - base[d];
+        fin = fin && is_finite(xv[d]);
+      }
+      if (k >= 0) cv = with_extra(a, k, cv);
+      fin = fin && is_finite(cv.x) && is_finite(cv.y);
+      if (k >= 0 && !fin) win_add_direct<T, DIM, NS>(a, cv, xv[0], xv[1], xv[DIM - 1], out);
+      if (k < 0 || !fin) {
+        zero_pair<T>(cv);
 #pragma unroll
         for (int d = 0; d < DIM; ++d) {
-          int prev = __shfl_up_sync(0xffffffffu, base[d], 1);
-          if (lane == 0) prev = cur[d];
-          differs = differs || prev != base[d];
+          dl[d] = i0[d] = 0;
+          xv[d] = (T)(NS / 2);
         }
-        const unsigned starts = cnt > 0 ? __ballot_sync(0xffffffffu, differs && lane < cnt) : 1u;
-        __syncwarp();
-        int j = 0;
-        do {  // one block (or the rest of one) per trip
-          if ((starts >> j) & 1u) {
-            if (cur[0] >= 0) win.flush(g, cur[0], cur[1], cur[2], lane, out);
-#pragma unroll
-            for (int d = 0; d < DIM; ++d) cur[d] = __shfl_sync(0xffffffffu, base[d], j);
-            if (DIM == 2) cur[2] = 0;
-          }
-          const unsigned later = j < 31 ? starts >> (j + 1) : 0u;
-          const int je = later != 0u ? min(j + __ffs(later), cnt) : cnt;
-          const T* sp = warp_slots + j * W::SLOT;
-          constexpr int U = DIM == 2 ? 4 : 2;
-          for (; j + U <= je; j += U, sp += U * W::SLOT) {
-#pragma unroll
-            for (int q = 0; q < U; ++q) win.add(sp + q * W::SLOT);
-          }
-#pragma unroll 1
-          for (; j < je; ++j, sp += W::SLOT) win.add(sp);
-        } while (j < cnt);
-        __syncwarp();
       }
+      T w[NS];
+      axis_weights<T, NS>(a, i0[0], xv[0], w);
+      Window<T, DIM, NS>::template stage<0>(my_slot, cv, w, dl[0]);
+      axis_weights<T, NS>(a, i0[1], xv[1], w);
+      Window<T, DIM, NS>::template stage<1>(my_slot, cv, w, dl[1]);
+      if constexpr (DIM == 3) {
+        axis_weights<T, NS>(a, i0[2], xv[2], w);
+        Window<T, DIM, NS>::template stage<2>(my_slot, cv, w, dl[2]);
+      }
+      // lane j starts a block when its block differs from point j - 1's
+      bool differs = false;
+#pragma unroll
+      for (int d = 0; d < DIM; ++d) {
+        int prev = __shfl_up_sync(0xffffffffu, base[d], 1);
+        if (lane == 0) prev = cur[d];
+        differs = differs || prev != base[d];
+      }
+      const unsigned starts = __ballot_sync(0xffffffffu, differs && lane < cnt);
+      __syncwarp();
+      int j = 0;
+      do {  // one block (or the rest of one) per trip
+        if ((starts >> j) & 1u) {
+          if (cur[0] >= 0) win.flush(g, cur[0], cur[1], cur[2], lane, out);
+#pragma unroll
+          for (int d = 0; d < DIM; ++d) cur[d] = __shfl_sync(0xffffffffu, base[d], j);
+          if (DIM == 2) cur[2] = 0;
+        }
+        const unsigned later = j < 31 ? starts >> (j + 1) : 0u;
+        const int je = later != 0u ? min(j + __ffs(later), cnt) : cnt;
+        const T* sp = warp_slots + j * W::SLOT;
+        win.add_run(sp, j, je, one_block);
+      } while (j < cnt);
+      __syncwarp();
     }
+    bool open = cur[0] >= 0;
+    if (one_block) open = send_sum<T, DIM, NS, NW>(win, cur, g, s_slots, warp, lane, out);
+    if (open) win.flush(g, cur[0], cur[1], cur[2], lane, out);
   }
   if constexpr (W::GROUP) __syncthreads();  // the list and counts are free for the next item
 }

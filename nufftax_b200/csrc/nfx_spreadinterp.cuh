@@ -46,6 +46,7 @@ struct PointArgs {
   int n_trans;
   int64_t grid_stride;  // complex elements per transform of the fine grid
   int win_part;         // window spread: points of one work item; 0: an item is a subproblem
+  int win_group;        // window spread: items that one takes together when their points share a block; 0: none
   int tma;              // 1: the interpolation stages interior tiles with the kernel's tensor map
   int* status;          // device status word (nonzero after a bounded wait gave up); set when tma = 1
   Geom g;
@@ -363,11 +364,20 @@ template <typename T>
 __device__ __forceinline__ int spread_items(const PointArgs<T>& a) {
   return a.win_part > 0 ? (int)((a.M + a.win_part - 1) / a.win_part) : *a.s.nsub;
 }
+// What spread_item needs of an item ahead of it (the ungrouped window spread).
+template <typename T, int DIM, int NS>
+__device__ __forceinline__ int item_keys(const PointArgs<T>& a, int item) {
+  if constexpr (DIM == 2 && sizeof(T) == 4)
+    return win_group_keys(a, item);
+  else
+    return 0;
+}
 template <typename T, int DIM, int NS, int NW>
 __device__ __forceinline__ void spread_item(const PointArgs<T>& a, const cplx_t<T>* __restrict__ c,
-                                            cplx_t<T>* __restrict__ fw, int item, unsigned char* smem_raw) {
+                                            cplx_t<T>* __restrict__ fw, int item, int ahead,
+                                            unsigned char* smem_raw) {
   if constexpr (WinShape<T, DIM, NS>::on) {
-    spread_window<T, DIM, NS, NW>(a, c, fw, item, smem_raw);
+    spread_window<T, DIM, NS, NW>(a, c, fw, item, ahead, smem_raw);
   } else {
     spread_subproblem_cells<T, DIM, NS, NW>(a, c, fw, item, smem_raw);
   }
@@ -384,7 +394,13 @@ __global__ void __launch_bounds__(NW * 32, spread_min_ctas<T, DIM, NS>()) k_spre
                                                     cplx_t<T>* __restrict__ fw) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const int nitems = spread_items(a);
-  for (int item = blockIdx.x; item < nitems; item += gridDim.x) spread_item<T, DIM, NS, NW>(a, c, fw, item, smem_raw);
+  int ahead = (int)blockIdx.x < nitems ? item_keys<T, DIM, NS>(a, blockIdx.x) : 0;
+  for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
+    const int keys = ahead;
+    const int next = item + gridDim.x;
+    if (next < nitems) ahead = item_keys<T, DIM, NS>(a, next);  // arrives while this item is spread
+    spread_item<T, DIM, NS, NW>(a, c, fw, item, keys, smem_raw);
+  }
 }
 
 // Plane-owner spread (3D, points sparser than cells).  The CTA stages up to
@@ -1089,7 +1105,9 @@ __global__ void __launch_bounds__(NW * 32) k_spread_batch(const BatchItem<T>* __
   for (int gi = blockIdx.x; gi < total; gi += gridDim.x) {
     const int p = batch_find(sub_prefix, nitems, gi);
     const BatchItem<T>& it = items[p];
-    spread_item<T, DIM, NS, NW>(it.a, (const cplx_t<T>*)it.src, (cplx_t<T>*)it.dst, gi - sub_prefix[p], smem_raw);
+    const int item = gi - sub_prefix[p];
+    spread_item<T, DIM, NS, NW>(it.a, (const cplx_t<T>*)it.src, (cplx_t<T>*)it.dst, item,
+                                item_keys<T, DIM, NS>(it.a, item), smem_raw);
     __syncthreads();
   }
 }
@@ -1436,7 +1454,9 @@ struct Launch {
   // this problem's items.
   static int64_t split_items(int64_t M_total, int ctas, PointArgs<T>& a) {
     if constexpr (WinShape<T, DIM, NS>::on) {
-      a.win_part = win_part_points(DIM, M_total, ctas);
+      const WinSplit w = win_split(DIM, SW, M_total, ctas, a.s.maxsub);
+      a.win_part = w.part;
+      a.win_group = w.group;
       return (a.M + a.win_part - 1) / a.win_part;
     } else {
       return a.s.max_subs;
@@ -1656,6 +1676,7 @@ PointArgs<T> make_args(const Geom& g, double beta, double kc, int64_t M, int n_t
   a.n_trans = n_trans;
   a.grid_stride = (int64_t)g.nf[0] * g.nf[1] * g.nf[2];
   a.win_part = 0;
+  a.win_group = 1;
   a.tma = 0;
   a.status = nullptr;
   a.g = g;
