@@ -127,7 +127,7 @@ size_t win_smem_bytes() {
 // points cost several times a 2D point and spread over more cells, so their items
 // may be smaller; sets too small to give every SM an item of the least size are
 // cut down to 64.
-// Groups (2D) reach the size of a subproblem, so that a crowded cell gets no more
+// Groups (2D complex64) reach the size of a subproblem, so that a crowded cell gets no more
 // partial sums than one tile per subproblem would send.  Float error of 2D points in
 // one cell, over the root of the sum of squares: 100 k 2.0e-7, 1M 4.2e-7, 4M 5.6e-7
 // (by shared-memory tiles 2.9e-7, 5.9e-7, 7.4e-7; every slice by itself 5.9e-7,
@@ -137,14 +137,14 @@ size_t win_smem_bytes() {
 struct WinSplit {
   int part, group;
 };
-inline WinSplit win_split(int dim, int warps, int64_t M, int ctas, int maxsub) {
+inline WinSplit win_split(int dim, bool grouped, int warps, int64_t M, int ctas, int maxsub) {
   const int64_t most = dim == 2 ? 1024 : kWinRound;
   const int64_t least = M < 256 * 148 ? 64 : (dim == 2 ? 512 : 128);
   const int64_t rounds = (M + ctas * most - 1) / (ctas * most);
-  int group = dim == 2 ? (int)(maxsub < most ? 1 : (maxsub > 4 * most ? 4 : maxsub / most)) : 1;
+  int group = grouped ? 1 : (int)(maxsub < most ? 1 : (maxsub > 4 * most ? 4 : maxsub / most));
   int64_t n = rounds > 0 ? (M + ctas * rounds - 1) / (ctas * rounds) : 1;
   n = ((n < least ? least : n) + 31) / 32 * 32;
-  if (dim == 2 && rounds <= 1 && maxsub > n) group = (int)(maxsub / n < 16 ? maxsub / n : 16);
+  if (!grouped && rounds <= 1 && maxsub > n) group = (int)(maxsub / n < 16 ? maxsub / n : 16);
   if (M * warps <= 512 * n) group = 0;
   return WinSplit{(int)n, group};
 }
@@ -483,8 +483,8 @@ __device__ __forceinline__ int win_group_points(const PointArgs<T>& a, int item,
   n = (int)min((int64_t)a.win_part * a.win_group, a.M - k);
   return k;
 }
-// The keys of that group's first and last point, in lanes 0 and 1.  An ungrouped
-// kernel loads them an item ahead; grouping waits for keys anyway.
+// The keys of that group's first and last point, in lanes 0 and 1, which an item of
+// an ungrouped kernel needs ahead.
 template <typename T>
 __device__ __forceinline__ int win_group_keys(const PointArgs<T>& a, int item) {
   if (a.win_group == 0) return 0;
@@ -499,10 +499,10 @@ __device__ __forceinline__ int win_group_keys(const PointArgs<T>& a, int item) {
 // each lane stages one point, and the warp adds the 32 one after another, flushing
 // the window whenever the block changes.  The next 32 points are fetched while the
 // current ones are added.
-// A crowded item: when all points of a group of `a.win_group` items lie in one
-// block, one of them takes the whole group and the others nothing, and its warps
-// send one window.  Which one rotates with the group's place in the grid-stride
-// order, so that each CTA gets its share.
+// A crowded item's points all lie in one block; its warps send one window.  Where a
+// block's points are contiguous, one item of a group of `a.win_group` whose points
+// share a block takes the whole group and the others nothing; which one rotates
+// with the group's place in the grid-stride order, so that each CTA gets its share.
 template <typename T, int DIM, int NS, int NW>
 __device__ __forceinline__ void spread_window(const PointArgs<T>& a, const cplx_t<T>* __restrict__ c,
                                               cplx_t<T>* __restrict__ fw, int item, int ahead,
@@ -515,16 +515,15 @@ __device__ __forceinline__ void spread_window(const PointArgs<T>& a, const cplx_
   const Geom& g = a.g;
   int k0 = item * a.win_part;
   int n = (int)min((int64_t)a.win_part, a.M - k0);
-  const int first_key = W::GROUP ? a.s.keys[k0] : 0, last_key = W::GROUP ? a.s.keys[k0 + n - 1] : 0;
-  const int ends = W::GROUP && DIM == 2 ? win_group_keys(a, item) : ahead;
-  const bool one_block =
-      a.win_group > 0 && (DIM == 3 ? same_block<T, DIM, NS>(a, first_key, last_key)  // groups of one
-                                   : same_block<T, DIM, NS>(a, __shfl_sync(0xffffffffu, ends, 0),
-                                                            __shfl_sync(0xffffffffu, ends, 1)));
-  if (one_block) {
-    k0 = win_group_points(a, item, n);
-    const unsigned members = (unsigned)((n + a.win_part - 1) / a.win_part);
-    if (item % a.win_group != (int)((unsigned)item / gridDim.x % members)) return;
+  bool one_block = false;
+  if constexpr (!W::GROUP) {  // a block's points are contiguous: the ends decide
+    one_block = a.win_group > 0 && same_block<T, DIM, NS>(a, __shfl_sync(0xffffffffu, ahead, 0),
+                                                          __shfl_sync(0xffffffffu, ahead, 1));
+    if (one_block) {
+      k0 = win_group_points(a, item, n);
+      const unsigned members = (unsigned)((n + a.win_part - 1) / a.win_part);
+      if (item % a.win_group != (int)((unsigned)item / gridDim.x % members)) return;
+    }
   }
   T* s_slots = reinterpret_cast<T*>(smem_raw);
   int* s_cnt = reinterpret_cast<int*>(s_slots + NT * W::SLOT);  // per block: points, then its list start
@@ -536,10 +535,10 @@ __device__ __forceinline__ void spread_window(const PointArgs<T>& a, const cplx_
   bool listed = false;
   if constexpr (W::GROUP) {
     const int per_bin = key_block<T, DIM, NS>(g, g.tile[0] * g.tile[1] * g.tile[2] - 1) + 1;  // blocks
-    const int bin0 = first_key >> a.s.cbits;
-    const int64_t span = (int64_t)((last_key >> a.s.cbits) - bin0 + 1) * per_bin;
+    const int bin0 = a.s.keys[k0] >> a.s.cbits;
+    const int64_t span = (int64_t)((a.s.keys[k0 + n - 1] >> a.s.cbits) - bin0 + 1) * per_bin;
     // more: few points per bin, no two of them are likely to share a block
-    listed = !one_block && span <= kWinBlocks && span >= 1;
+    listed = span <= kWinBlocks && span >= 1;
     if (listed) {
       const int nblk = (int)span;
       const int cmask = (1 << a.s.cbits) - 1;
@@ -571,10 +570,16 @@ __device__ __forceinline__ void spread_window(const PointArgs<T>& a, const cplx_
         run += v;
       }
       __syncthreads();
+      bool first = true;  // whether the thread's points lie in the first block that has any
 #pragma unroll
-      for (int i = 0; i < PER; ++i)
-        if (key[i] >= 0) s_list[s_cnt[key[i]] + rank[i]] = (unsigned short)(i * NT + threadIdx.x);
-      __syncthreads();
+      for (int i = 0; i < PER; ++i) {
+        if (key[i] >= 0) {
+          const int at = s_cnt[key[i]];
+          first = first && at == 0;
+          s_list[at + rank[i]] = (unsigned short)(i * NT + threadIdx.x);
+        }
+      }
+      one_block = __syncthreads_and(first) && a.win_group > 0;
     }
   }
   // ---- the warp's slice of the list, per transform ----

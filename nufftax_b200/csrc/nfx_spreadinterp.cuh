@@ -1454,7 +1454,7 @@ struct Launch {
   // this problem's items.
   static int64_t split_items(int64_t M_total, int ctas, PointArgs<T>& a) {
     if constexpr (WinShape<T, DIM, NS>::on) {
-      const WinSplit w = win_split(DIM, SW, M_total, ctas, a.s.maxsub);
+      const WinSplit w = win_split(DIM, WinShape<T, DIM, NS>::GROUP, SW, M_total, ctas, a.s.maxsub);
       a.win_part = w.part;
       a.win_group = w.group;
       return (a.M + a.win_part - 1) / a.win_part;
