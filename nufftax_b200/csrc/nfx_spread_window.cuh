@@ -44,7 +44,12 @@
 namespace nfx {
 
 constexpr int kWinRound = 2048;   // most points of a work item (16-bit list entries)
-constexpr int kWinBlocks = 1024;  // most blocks (of all its bins) an item is grouped by
+// Most blocks (of all its bins) an item is grouped by.  3D: what 2048 points span at
+// half a point a block, below which grouping saves few reds.  With 1024, sparse sets
+// on large grids went ungrouped: ns 8, 600 k points on 288^3 1770 us (grouped 1011,
+// the plane-owner spread 1052), on 320^3 2008 (1271, 1353), 4M on 512^3 11740 (6153,
+// 8400), 1M 4611 (3893, 6726); 300 points to 1M on 64^3 to 256^3 are unchanged.
+constexpr int win_blocks(int dim) { return dim == 3 ? 4096 : 1024; }
 
 // Block and lane layout per dimension and width.  2D: lane = (x, row group),
 // LW x positions times H row groups of RL rows each.  3D: a lane owns NCOL
@@ -115,18 +120,17 @@ constexpr int win_warps() {
 template <typename T, int DIM, int NS>
 size_t win_smem_bytes() {
   return (size_t)win_warps<T, DIM, NS>() * 32 * WinShape<T, DIM, NS>::SLOT * sizeof(T) +
-         (WinShape<T, DIM, NS>::GROUP ? kWinBlocks * sizeof(int) + kWinRound * sizeof(unsigned short) : 0);
+         (WinShape<T, DIM, NS>::GROUP ? win_blocks(DIM) * sizeof(int) + kWinRound * sizeof(unsigned short) : 0);
 }
 
 // Work items of a spread of M points on `ctas` resident CTAs: points of one item,
 // and the items of a group that one CTA takes when their points share a block.
 // The items are equal, so as many as the CTAs take in whole rounds, of at most
-// kWinRound points (2D: 1024; 4M clustered points 146 us, 159 with 2048, whose
-// four rounds end unevenly).  The least size bounds the partial sums a crowded
-// cell gets (each slice of a warp adds its own, and their float rounding).  3D
-// points cost several times a 2D point and spread over more cells, so their items
-// may be smaller; sets too small to give every SM an item of the least size are
-// cut down to 64.
+// kWinRound points (2D: 1024; 2048 gives 4M clustered points on 1024^2 167 us for
+// 161, on 4096^2 255 for 202, uniform 4M 148 for 153).  They go down to 32 points (a
+// warp then stages a few): with at least 64, 1 k points on 1024^2 15.4 us, 13.3 with
+// 32, 3D on 64^3 35.7 and 25.5; with at least 512 in 2D above 37,888 points (74 items
+// for 148 SMs) 38 k points 31.8 us, 21.5 now, 100 k clustered 35.8 and 23.6.
 // Groups (2D complex64) reach the size of a subproblem, so that a crowded cell gets no more
 // partial sums than one tile per subproblem would send.  Float error of 2D points in
 // one cell, over the root of the sum of squares: 100 k 2.0e-7, 1M 4.2e-7, 4M 5.6e-7
@@ -139,11 +143,10 @@ struct WinSplit {
 };
 inline WinSplit win_split(int dim, bool grouped, int warps, int64_t M, int ctas, int maxsub) {
   const int64_t most = dim == 2 ? 1024 : kWinRound;
-  const int64_t least = M < 256 * 148 ? 64 : (dim == 2 ? 512 : 128);
   const int64_t rounds = (M + ctas * most - 1) / (ctas * most);
   int group = grouped ? 1 : (int)(maxsub < most ? 1 : (maxsub > 4 * most ? 4 : maxsub / most));
   int64_t n = rounds > 0 ? (M + ctas * rounds - 1) / (ctas * rounds) : 1;
-  n = ((n < least ? least : n) + 31) / 32 * 32;
+  n = (n + 31) / 32 * 32;
   if (!grouped && rounds <= 1 && maxsub > n) group = (int)(maxsub / n < 16 ? maxsub / n : 16);
   if (M * warps <= 512 * n) group = 0;
   return WinSplit{(int)n, group};
@@ -527,7 +530,7 @@ __device__ __forceinline__ void spread_window(const PointArgs<T>& a, const cplx_
   }
   T* s_slots = reinterpret_cast<T*>(smem_raw);
   int* s_cnt = reinterpret_cast<int*>(s_slots + NT * W::SLOT);  // per block: points, then its list start
-  unsigned short* s_list = reinterpret_cast<unsigned short*>(s_cnt + kWinBlocks);
+  unsigned short* s_list = reinterpret_cast<unsigned short*>(s_cnt + win_blocks(DIM));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   T* my_slot = s_slots + (warp * 32 + lane) * W::SLOT;
   const T* warp_slots = s_slots + warp * 32 * W::SLOT;
@@ -537,8 +540,8 @@ __device__ __forceinline__ void spread_window(const PointArgs<T>& a, const cplx_
     const int per_bin = key_block<T, DIM, NS>(g, g.tile[0] * g.tile[1] * g.tile[2] - 1) + 1;  // blocks
     const int bin0 = a.s.keys[k0] >> a.s.cbits;
     const int64_t span = (int64_t)((a.s.keys[k0 + n - 1] >> a.s.cbits) - bin0 + 1) * per_bin;
-    // more: few points per bin, no two of them are likely to share a block
-    listed = span <= kWinBlocks && span >= 1;
+    // more: sparse points, few of them share a block
+    listed = span <= win_blocks(DIM) && span >= 1;
     if (listed) {
       const int nblk = (int)span;
       const int cmask = (1 << a.s.cbits) - 1;
