@@ -1097,9 +1097,16 @@ __device__ __forceinline__ int batch_find(const int* __restrict__ prefix, int n,
   return lo;
 }
 
+// CTAs per SM the batched spread's registers must allow for (0: the compiler's
+// choice): as the plain spread's where a window exists.
+template <typename T, int DIM, int NS>
+constexpr int batch_min_ctas() {
+  return WinShape<T, DIM, NS>::on ? spread_min_ctas<T, DIM, NS>() : 0;
+}
+
 template <typename T, int DIM, int NS, int NW>
-__global__ void __launch_bounds__(NW * 32) k_spread_batch(const BatchItem<T>* __restrict__ items, int nitems,
-                                                          const int* __restrict__ sub_prefix) {
+__global__ void __launch_bounds__(NW * 32, batch_min_ctas<T, DIM, NS>())
+    k_spread_batch(const BatchItem<T>* __restrict__ items, int nitems, const int* __restrict__ sub_prefix) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const int total = sub_prefix[nitems];
   for (int gi = blockIdx.x; gi < total; gi += gridDim.x) {
@@ -1560,6 +1567,17 @@ template <typename T, int DIM, int NS>
 struct BatchLaunch {
   static constexpr int NW = warps_per_cta(sizeof(T), DIM, NS);
   static constexpr int SW = win_warps<T, DIM, NS>();
+  // CTAs of the batched window spread that the GPU holds at a time (its shared
+  // memory does not depend on the problem).
+  static int window_ctas() {
+    int grid = 0;
+    if constexpr (WinShape<T, DIM, NS>::on) {
+      if (kernel_grid(reinterpret_cast<const void*>(k_spread_batch<T, DIM, NS, SW>), SW * 32,
+                      win_smem_bytes<T, DIM, NS>(), INT32_MAX, grid) != cudaSuccess)
+        grid = 0;  // the launch reports it
+    }
+    return std::max(grid, 1);
+  }
   static cudaError_t spread(const void* items, int n, const int* prefix, int64_t max_subs, size_t smem,
                             cudaStream_t st) {
     int grid = 0;
@@ -1613,11 +1631,10 @@ size_t spread_smem_dim(int ns, const Geom& g) {
 // Work items of one problem of a batched spread (Launch::split_items).
 template <typename T, int DIM>
 int64_t split_spread_items(int ns, int64_t M_total, PointArgs<T>& a) {
-  const int ctas = num_sms() * (DIM == 2 ? 4 : 2);
   switch (ns) {
 #define NFX_CASE(N) \
   case N:           \
-    return Launch<T, DIM, N>::split_items(M_total, ctas, a);
+    return Launch<T, DIM, N>::split_items(M_total, BatchLaunch<T, DIM, N>::window_ctas(), a);
     NFX_CASE(2) NFX_CASE(4) NFX_CASE(6) NFX_CASE(8) NFX_CASE(10) NFX_CASE(12) NFX_CASE(14) NFX_CASE(16)
 #undef NFX_CASE
     default:
