@@ -401,7 +401,7 @@ static void make_layout(const nfx_opts& o, const Geom& g, int64_t M, SortLayout&
   L.ncell = g.tile[0] * g.tile[1] * g.tile[2];
   radix_plan(g.nbins, L.ncell, L.cbits, L.bits, L.npass, L.dbits);
   const int64_t B = (int64_t)1 << L.dbits;
-  L.chunk = radix_chunk(M);
+  L.chunk = radix_chunk(M, L.dbits);
   L.nchunks = (int)((M + L.chunk - 1) / L.chunk);
   L.maxsub = o.max_subproblem > 0 ? o.max_subproblem : auto_max_subproblem(o.dim, M);
   L.max_subs = g.nbins + (M + L.maxsub - 1) / L.maxsub;
@@ -416,7 +416,7 @@ static void make_layout(const nfx_opts& o, const Geom& g, int64_t M, SortLayout&
   L.off_vals_tmp = take((size_t)M * 4);
   L.off_keys_sorted = take((size_t)M * 4);
   L.off_perm = take((size_t)M * 4);
-  L.off_counts = take((size_t)radix_count_rows(M) * B * 4);
+  L.off_counts = take((size_t)radix_count_rows(M, L.dbits) * B * 4);
   L.off_totals = take((size_t)B * 4);
   L.off_bin_start = take((size_t)(g.nbins + 1) * 4);
   L.off_sub_bin = take((size_t)L.max_subs * 4);

@@ -74,10 +74,10 @@ struct SortView {
 };
 
 void radix_plan(int nbins, int ncell, int& cbits, int& bits, int& npass, int& dbits);
-// Elements per chunk of a sort of M points, and the rows of its count matrix
-// (at least one per chunk).
-int radix_chunk(int64_t M);
-int radix_count_rows(int64_t M);
+// Elements per chunk of a sort of M points by digits of dbits bits, and the rows of
+// its count matrix (at least one per chunk).
+int radix_chunk(int64_t M, int dbits);
+int radix_count_rows(int64_t M, int dbits);
 // out[i] = bin of point i (composite key / cells per tile)
 cudaError_t bin_keys_of(const SortLayout& L, const int* K, int* out, cudaStream_t st);
 

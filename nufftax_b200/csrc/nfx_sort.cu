@@ -89,6 +89,12 @@ constexpr int kRadixThreads = 256;
 constexpr int kRadixItems = 16;
 constexpr int kRadixItemsSmall = 4;
 constexpr int64_t kRadixSmallM = 148 * 2 * kRadixThreads * kRadixItemsSmall;  // two CTAs an SM
+// 11-bit digits clear and scan 16384 counters a chunk: with short chunks a sort of
+// 300 k points takes 85 us (long 75), of 200 k 79 (75), of 100 k 60 (75), and sorts
+// that run side by side pay for all of it (16 of 10 k to 200 k points with their
+// transforms, replayed: 275 us with short chunks up to 303 k, 247 with this limit, 240
+// without any).  10 bits: 300 k points 52 us, long 62.
+constexpr int64_t kRadixSmallM11 = kRadixSmallM / 4;
 
 // ---- (1) composite keys + the first digit's per-chunk counts ---------------
 // One CTA per chunk of consecutive points: K = bin << cbits | cell
@@ -680,15 +686,19 @@ void radix_plan(int nbins, int ncell, int& cbits, int& bits, int& npass, int& db
   dbits = (bits + npass - 1) / npass;
 }
 
-int radix_chunk(int64_t M) { return kRadixThreads * (M <= kRadixSmallM ? kRadixItemsSmall : kRadixItems); }
+static int64_t small_sort(int dbits) { return dbits >= 11 ? kRadixSmallM11 : kRadixSmallM; }
 
-// Just above kRadixSmallM the longer chunks need fewer rows than just below; the
-// reserve then shrinks more slowly than the per-point arrays grow, so that a
-// workspace that fits M points fits every smaller M.
-int radix_count_rows(int64_t M) {
-  const int64_t rows = (M + radix_chunk(M) - 1) / radix_chunk(M);
-  const int64_t reserve = kRadixSmallM / (kRadixThreads * kRadixItemsSmall) - (M - kRadixSmallM) / 4096;
-  return (int)(M > kRadixSmallM && reserve > rows ? reserve : rows);
+int radix_chunk(int64_t M, int dbits) {
+  return kRadixThreads * (M <= small_sort(dbits) ? kRadixItemsSmall : kRadixItems);
+}
+
+// Just above small_sort the longer chunks need fewer rows than just below: the rows
+// stay, so that the workspace does not shrink there.  (It does, by about 12 KB, where
+// the default subproblem size doubles, at 3.03M and 6.06M points in 1D and 2D.)
+int radix_count_rows(int64_t M, int dbits) {
+  const int64_t rows = (M + radix_chunk(M, dbits) - 1) / radix_chunk(M, dbits), limit = small_sort(dbits);
+  const int64_t least = M > limit ? limit / (kRadixThreads * kRadixItemsSmall) : 0;
+  return (int)(rows > least ? rows : least);
 }
 
 cudaError_t bin_keys_of(const SortLayout& L, const int* K, int* out, cudaStream_t st) {

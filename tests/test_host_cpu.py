@@ -342,3 +342,22 @@ def test_grid_stride_walk_ends_at_the_largest_m(n):
         visited, outside = ctypes.c_int64(), ctypes.c_int64()
         assert lib.nfx_selftest_positions(n, first, stride, ctypes.byref(visited), ctypes.byref(outside)) == 0
         assert (visited.value, outside.value) == ((n - 1 - first) // stride + 1, 0)
+
+
+@pytest.mark.parametrize("precision", [_lib.NFX_F32, _lib.NFX_F64])
+@pytest.mark.parametrize("nf", [(2_097_152,), (512, 486), (2048, 2048), (96, 90, 64)])
+def test_sort_workspace_grows_with_m(nf, precision):
+    """Up to the first doubling of the default subproblem size (3,031,040 points) a
+    workspace that fits M points fits every smaller M, also where the sort's chunks
+    change."""
+    from nufftax_b200._plan import make_opts
+
+    lib = _lib.load()
+    o = make_opts(precision, nf, nb.compute_kernel_params(1e-6), True)
+    edges = [1, 1024, 4096, 75_776, 75_776 + 4096, 303_104, 303_104 + 4096, 1_212_416, 3_031_000]
+    last = 0
+    for M in sorted({e + d for e in edges for d in (-1, 0, 1, 2)}):
+        n = c_size_t(0)
+        assert lib.nfx_sort_workspace_bytes(byref(o), M, byref(n)) == 0
+        assert n.value >= last, M
+        last = n.value
