@@ -394,11 +394,18 @@ class TransformPlan:
     def sort(self, coords) -> PointSort:
         return sort_cache.get(coords, self.nf, self.kp, True, self.opts)
 
+    def _call_by_call(self, *names: str) -> bool:
+        """Whether the named calls are made one by one: a recorder times one of
+        them, or the stream captures (a captured FFT takes its own work area)."""
+        if recording(*names):
+            return True
+        with on_device(self.device):
+            return torch.cuda.is_current_stream_capturing()
+
     def type1(self, ps: PointSort, c: torch.Tensor, sign: int) -> torch.Tensor:
         """Strengths (n_trans, M) at sorted points -> modes: spread, FFT, deconvolve."""
         c = ps._check_strengths(c)
-        if recording() or torch.cuda.is_current_stream_capturing():
-            # call by call: each is timed, and a captured FFT takes its own work area
+        if self._call_by_call("nfx_spread_sorted", "nfx_fft", "nfx_deconv_shuffle"):
             fw = ps.spread(c)
             fft_inplace(fw, self.dim, sign)
             return deconv_shuffle(fw, self.n_modes, self.kp)
@@ -415,7 +422,7 @@ class TransformPlan:
     def type2_grid(self, f: torch.Tensor, sign: int) -> torch.Tensor:
         """Modes (n_trans, ..) -> the fine grid to interpolate: deconvolve, zero-pad, FFT."""
         f = f.contiguous()
-        if recording() or torch.cuda.is_current_stream_capturing():
+        if self._call_by_call("nfx_deconv_pad", "nfx_fft"):
             return fft_inplace(deconv_pad(f, self.nf, self.kp), self.dim, sign)
         nt = f.shape[0]
         fw = torch.empty((nt,) + self.grid_shape, dtype=f.dtype, device=self.device)

@@ -52,9 +52,10 @@ def record(only=None):
         _state.rec = prev
 
 
-def recording() -> bool:
-    """Whether a `record()` is active on this thread."""
-    return getattr(_state, "rec", None) is not None
+def recording(*names: str) -> bool:
+    """Whether a `record()` on this thread takes any of the named calls."""
+    rec = getattr(_state, "rec", None)
+    return rec is not None and (rec.only is None or not rec.only.isdisjoint(names))
 
 
 class span:

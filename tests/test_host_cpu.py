@@ -361,3 +361,18 @@ def test_sort_workspace_grows_with_m(nf, precision):
         assert lib.nfx_sort_workspace_bytes(byref(o), M, byref(n)) == 0
         assert n.value >= last, M
         last = n.value
+
+
+def test_a_recorder_of_one_call_leaves_the_others_alone():
+    """recording(names) tells whether a recorder on this thread takes any of them:
+    the transforms join their calls unless one of them is timed."""
+    from nufftax_b200 import profiling
+
+    type1 = ("nfx_spread_sorted", "nfx_fft", "nfx_deconv_shuffle")
+    type2 = ("nfx_deconv_pad", "nfx_fft")
+    assert not profiling.recording(*type1)
+    with profiling.record(only=["nfx_spread_sorted"]):
+        assert profiling.recording(*type1) and not profiling.recording(*type2)
+    with profiling.record():
+        assert profiling.recording(*type1) and profiling.recording(*type2)
+    assert not profiling.recording(*type2)
