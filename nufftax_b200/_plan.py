@@ -63,6 +63,12 @@ def on_device(device: torch.device):
     return torch.cuda.device(device)
 
 
+def plain(t: torch.Tensor) -> torch.Tensor:
+    """t as its memory should read for a kernel: contiguous, and no lazy conjugate or
+    negative view (whose memory holds other values than the tensor stands for)."""
+    return t.resolve_conj().resolve_neg().contiguous()
+
+
 def ptr(t: torch.Tensor | None):
     return None if t is None else c_void_p(t.data_ptr())
 
@@ -136,7 +142,7 @@ class PointSort:
             raise ValueError("coords and nf must have 1, 2 or 3 axes")
         self.device = coords[0].device
         self.precision = precision_of(coords[0].dtype)
-        self.coords = [c.contiguous() for c in coords]
+        self.coords = [plain(c) for c in coords]
         self.M = int(self.coords[0].shape[0])
         for c in self.coords:
             require_cuda(c, "coordinates")
@@ -201,13 +207,13 @@ class PointSort:
         if c.dtype != complex_dtype(self.precision) or c.shape[-1] != self.M or c.ndim != 2:
             raise ValueError(f"strengths must be (n_trans, {self.M}) {complex_dtype(self.precision)}")
         require_cuda(c, "strengths")
-        return c.contiguous()
+        return plain(c)
 
     def _check_grid(self, fw: torch.Tensor) -> torch.Tensor:
         if fw.dtype != complex_dtype(self.precision) or tuple(fw.shape[1:]) != self.grid_shape:
             raise ValueError(f"grid must be (n_trans, {self.grid_shape}) {complex_dtype(self.precision)}")
         require_cuda(fw, "grid")
-        return fw.contiguous()
+        return plain(fw)
 
     # -- passes ------------------------------------------------------------
     def spread(self, c: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
@@ -421,7 +427,7 @@ class TransformPlan:
 
     def type2_grid(self, f: torch.Tensor, sign: int) -> torch.Tensor:
         """Modes (n_trans, ..) -> the fine grid to interpolate: deconvolve, zero-pad, FFT."""
-        f = f.contiguous()
+        f = plain(f)
         if self._call_by_call("nfx_deconv_pad", "nfx_fft"):
             return fft_inplace(deconv_pad(f, self.nf, self.kp), self.dim, sign)
         nt = f.shape[0]
@@ -516,7 +522,7 @@ def deconv_pad(f: torch.Tensor, nf: Sequence[int], kp: KernelParams, out: torch.
     """(n_trans, n_d..n_1) CMCL modes -> zero-padded deconvolved (n_trans, nf_d..nf_1)."""
     dim = len(nf)
     precision = precision_of(f.dtype)
-    f = f.contiguous()
+    f = plain(f)
     n_modes = tuple(reversed(f.shape[-dim:]))
     fs = _facs(nf, n_modes, kp, precision, f.device)
     if out is None:

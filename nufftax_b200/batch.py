@@ -26,7 +26,7 @@ from typing import Sequence
 import torch
 
 from . import _lib
-from ._plan import complex_dtype, factors, precision_of, ptr, real_dtype, stream_of
+from ._plan import complex_dtype, factors, plain, precision_of, ptr, real_dtype, stream_of
 from .grid import compute_grid_size
 from .kernel import compute_kernel_params
 
@@ -55,7 +55,7 @@ class BatchPlan:
         self.eps = eps
         self.isign1, self.isign2 = int(isign_type1), int(isign_type2)
         self.kp = compute_kernel_params(eps, upsampfac)
-        self.points = [[c.to(self.rdt).contiguous() for c in pts] for pts in points]
+        self.points = [[plain(c.to(self.rdt)) for c in pts] for pts in points]
         for pts in self.points:
             if len(pts) != self.dim or any(not c.is_cuda for c in pts):
                 raise ValueError("every problem needs dim CUDA coordinate tensors")

@@ -34,7 +34,7 @@ from ctypes import byref, c_size_t, c_void_p
 
 from . import _lib
 from ._plan import (PointSort, _facs, complex_dtype, deconv_pad, deconv_shuffle, fft_inplace, make_opts, precision_of,
-                    ptr, real_dtype)
+                    plain, ptr, real_dtype)
 from .grid import compute_grid_size
 from .kernel import compute_kernel_params
 from .transforms import _fft_sign_type1, _fft_sign_type2, _type3_forward
@@ -249,9 +249,9 @@ class NufftServer:
     def _run_one_call(self, req: Request, slot: _Slot):
         """Type 1/2 on unshared points: one library call (sort, spread or interp,
         FFT, deconvolution) on the slot's pooled workspace and a pooled grid."""
-        c = req.strengths.contiguous()
+        c = plain(req.strengths)
         precision = precision_of(c.dtype)
-        xs = [x.contiguous() for x in req.coords]
+        xs = [plain(x) for x in req.coords]
         if len(xs) != req.dim or any(x.dtype != real_dtype(precision) or x.shape != (req.M,) for x in xs):
             raise ValueError(f"coordinates must be {req.dim} tensors of shape ({req.M},), {real_dtype(precision)}")
         want = (req.M,) if req.kind == 1 else tuple(reversed(req.n_modes))
@@ -318,9 +318,9 @@ class NufftServer:
         fields and library options (raises for a malformed request)."""
         if req.make_inputs is not None:
             req.coords, req.strengths, req.targets = req.make_inputs(self.device)
-        c = req.strengths.contiguous()
+        c = plain(req.strengths)
         precision = precision_of(c.dtype)
-        xs = [x.contiguous() for x in req.coords]
+        xs = [plain(x) for x in req.coords]
         if len(xs) != req.dim or any(x.dtype != real_dtype(precision) or x.shape != (req.M,) for x in xs):
             raise ValueError(f"coordinates must be {req.dim} tensors of shape ({req.M},), {real_dtype(precision)}")
         want = (req.M,) if req.kind == 1 else tuple(reversed(req.n_modes))

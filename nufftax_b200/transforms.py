@@ -45,7 +45,7 @@ import torch
 import torch.autograd.forward_ad as _fwad
 
 from . import _lib
-from ._plan import (_facs, complex_dtype, make_opts, on_device, precision_of, ptr, real_dtype, sort_launches,
+from ._plan import (_facs, complex_dtype, make_opts, on_device, plain, precision_of, ptr, real_dtype, sort_launches,
                     stream_of, transform_plan)
 from .profiling import span
 from .grid import compute_grid_size
@@ -169,7 +169,7 @@ def _type1_coord_grad(c2, G, n_modes, eps, isign, uf_t, need_c, need_x, coords):
     grid, then one fused ES-derivative pass over the points."""
     pl = transform_plan(n_modes, eps, uf_t, precision_of(G.dtype), G.device)
     H = pl.type2_grid(G, -_fft_sign_type1(isign))
-    return pl.sort(coords).spread_grad(c2.contiguous(), H, need_c, need_x)
+    return pl.sort(coords).spread_grad(c2, H, need_c, need_x)
 
 
 def _type2_plan(f2, eps, uf):
@@ -189,7 +189,7 @@ def _type2_coord_grad(f2, G, n_modes, eps, isign, uf, need_x, coords):
     interpolation on it."""
     pl = _type2_plan(f2, eps, uf)
     fw = pl.type2_grid(f2, _fft_sign_type2(isign))
-    return pl.sort(coords).interp_grad(fw, G.contiguous(), need_x)
+    return pl.sort(coords).interp_grad(fw, G, need_x)
 
 
 def _split_stack(F, nt, first):
@@ -488,9 +488,9 @@ def _type3_forward(src: list[torch.Tensor], c2: torch.Tensor, tgt: list[torch.Te
     def parr(ts):
         return arr(*([t.data_ptr() for t in ts] + [None] * (3 - len(ts))))
 
-    src = [a.contiguous() for a in src]
-    tgt = [a.contiguous() for a in tgt]
-    c2 = c2.contiguous()
+    src = [plain(a) for a in src]
+    tgt = [plain(a) for a in tgt]
+    c2 = plain(c2)
     # our kernels: min / max of every array, the scalars, both sorts, spread, zero-pad, interp
     launches = lambda: (2 + sort_launches(opts, M, type3=True) + 2  # noqa: E731 (evaluated only when recording)
                         + sort_launches(make_opts(precision, nf_in, kp, prenorm=True), K, type3=True) + 1)
