@@ -1287,15 +1287,18 @@ __global__ void __launch_bounds__(NW * 32, grad_min_ctas<T, DIM, NS>()) k_grad(c
   T* douts[3] = {dx, dy, dz};
   for (int sidx = blockIdx.x; sidx < nsub; sidx += gridDim.x) {
     const int b = a.s.sub_bin[sidx];
-    // 3D, a lane group per point where the bin holds fewer points than cells: a
-    // warp's 32 points are then many cells apart and their footprint reads
-    // conflict.  In denser bins neighbouring threads read nearly the same cells,
-    // and a thread per point is the faster one.  Thread -> group, us, complex64 ns
-    // 8: 8M on 256^3 (0.5 a cell) 2592 -> 2176, 1M on 192x225x256 583 -> 539; but
-    // 4M on 128^3 (1.9 a cell) 881 -> 946, 1M clustered 254 -> 311.  Widths that
-    // fill their lane groups only (ns 6 398 -> 445, complex128 ns 10 315 -> 381).
-    if constexpr (DIM == 3 && (NS == 4 || NS == 8)) {
-      if (a.s.bin_start[b + 1] - a.s.bin_start[b] < g.tile[0] * g.tile[1] * g.tile[2]) {
+    // 3D width 8, a lane group per point where the bin holds fewer points than cells
+    // (and enough for four warps): a warp's 32 points are then many cells apart and
+    // their footprint reads conflict.  In denser bins neighbouring threads read nearly
+    // the same cells, and a thread per point is the faster one.  Thread -> group, us,
+    // complex64: 8M on 256^3 (0.5 a cell) 2592 -> 2176, 1M on 192x225x256 583 -> 539;
+    // but 4M on 128^3 (1.9 a cell) 881 -> 946, 1M clustered 254 -> 311, 100 k on 128^3
+    // (98 a bin) 138 -> 142.  Other widths lose: ns 4, 4M on 256^3 520 -> 674 (the group
+    // form also takes its registers from 80 to 99), ns 6 398 -> 445, complex128 ns 10
+    // 315 -> 381.
+    if constexpr (DIM == 3 && NS == 8) {
+      const int in_bin = a.s.bin_start[b + 1] - a.s.bin_start[b];
+      if (in_bin >= 128 && in_bin < g.tile[0] * g.tile[1] * g.tile[2]) {
         if (!grad_group<T, NS, NW>(a, G, V, out_interp, dx, dy, dz, sidx, smem_raw, ts)) return;
         continue;
       }
