@@ -1060,8 +1060,18 @@ __device__ __forceinline__ void interp_subproblem(const PointArgs<T>& a, const c
   }
 }
 
+// CTAs per SM the interpolation's registers must allow for (0: the compiler's
+// choice).  The polynomial weights gave complex128 in 2D 148 registers and more from
+// ns 12, one CTA an SM, which shows where few points a bin wait for their tiles: ns
+// 14 on 512^2, us by exp/sqrt, one CTA, two: 5 k points 19.5, 25.6, 17.4; 500 k 107,
+// 100, 82; 3M 506, 444, 363 (the spills it costs are small beside that).
+template <typename T, int DIM, int NS, int MODE>
+constexpr int interp_min_ctas() {
+  return sizeof(T) == 8 && DIM == 2 && NS >= 12 && MODE == NFX_PER_POINT_THREAD ? 2 : 0;
+}
+
 template <typename T, int DIM, int NS, int NW, int MODE>
-__global__ void __launch_bounds__(NW * 32) k_interp(PointArgs<T> a, const cplx_t<T>* __restrict__ fw,
+__global__ void __launch_bounds__(NW * 32, interp_min_ctas<T, DIM, NS, MODE>()) k_interp(PointArgs<T> a, const cplx_t<T>* __restrict__ fw,
                                                     cplx_t<T>* __restrict__ cout, const __grid_constant__ CUtensorMap tmap) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t mbar;
