@@ -129,10 +129,14 @@ bool interp_tile_map(CUtensorMap_st* map, size_t real_bytes, int dim, const Geom
   return res == CUDA_SUCCESS;
 }
 
+// Dynamic shared memory up to this needs no attribute: a kernel's static arrays (a
+// few hundred bytes) count towards the default limit of 48 KB too.
+constexpr size_t kSmemNoAttribute = 40 * 1024;
+
 cudaError_t ensure_smem(const void* fn, size_t smem) {
   static std::mutex mu;
   static std::map<std::pair<const void*, int>, size_t> done;
-  if (smem <= 48 * 1024) return cudaSuccess;
+  if (smem <= kSmemNoAttribute) return cudaSuccess;
   int dev = 0;
   cudaGetDevice(&dev);
   std::lock_guard<std::mutex> lk(mu);
@@ -171,7 +175,7 @@ cudaError_t kernel_grid(const void* fn, int threads, size_t smem, int64_t max_wo
       per_sm = it->second;
     } else {
       auto ak = std::make_pair(fn, dev);
-      if (smem > 48 * 1024 && smem_attr[ak] < smem) {
+      if (smem > kSmemNoAttribute && smem_attr[ak] < smem) {
         cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
         smem_attr[ak] = smem;
