@@ -383,9 +383,13 @@ __device__ __forceinline__ void spread_item(const PointArgs<T>& a, const cplx_t<
   }
 }
 
-// CTAs per SM the spread's registers allow for: the window accumulators.
+// CTAs per SM the spread's registers must allow for (0: the compiler's choice): the
+// window's accumulators take them, a tile spread runs on its residency (1D, 2M points,
+// ns 8: 177 us unbounded, 187 with the window's bounds, which let it have 56 registers
+// instead of 40).
 template <typename T, int DIM, int NS>
 constexpr int spread_min_ctas() {
+  if (!WinShape<T, DIM, NS>::on) return 0;
   return DIM == 3 || sizeof(T) == 8 ? 2 : (NS <= 8 ? 4 : 3);
 }
 
@@ -1273,9 +1277,11 @@ __device__ __forceinline__ bool grad_group(const PointArgs<T>& a, const cplx_t<T
 // ---------------------------------------------------------------------------
 // CTAs per SM the gradient pass's registers must allow for (0: the compiler's
 // choice).  1D complex128 at small widths runs on its residency: ns 6, 2M points,
-// 107 us with four CTAs, 116 with three.
+// 107 us with four CTAs, 116 with three; 3D complex64 at widths 4 and 6 too (ns 6, 4M
+// points on 256^3: 718 us with three, 937 with two).
 template <typename T, int DIM, int NS>
 constexpr int grad_min_ctas() {
+  if (sizeof(T) == 4 && DIM == 3 && (NS == 4 || NS == 6)) return 3;
   return sizeof(T) == 8 && DIM == 1 && NS <= 6 ? (NS == 2 ? 5 : 4) : 0;
 }
 
