@@ -248,10 +248,12 @@ struct Window<T, 2, NS> {
   }
   PT acc[W::RL];  // complex cells of this lane's rows
   int xo, yo;     // this lane's entries of a slot
+  int zeros_at;   // x offset around which this lane's own slot holds zeros; -1: none
 
   __device__ __forceinline__ explicit Window(int lane) {
     xo = 2 * (lane % W::LW);
     yo = W::YO + (lane / W::LW) * W::RS;
+    zeros_at = -1;
     clear();
   }
   __device__ __forceinline__ PT& cell(int i) { return acc[i]; }
@@ -259,12 +261,27 @@ struct Window<T, 2, NS> {
 #pragma unroll
     for (int i = 0; i < W::RL; ++i) acc[i] = pair_of((T)0, (T)0);
   }
-  // Axis D's weights (times the strength on x) at offset dl of its section,
-  // zeros in the rest of it.
+  // Axis D's weights (times the strength on x) at offset dl of its section, zeros
+  // in the rest of it: on x they are still there from the lane's last point while
+  // the offset stays (8M clustered points 269 -> 261 us, sparse sets as before), a row block's
+  // offset is always 0.
   template <int D>
-  static __device__ __forceinline__ void stage(T* sp, CT cv, const T (&w)[NS], int dl) {
+  __device__ __forceinline__ void stage(T* sp, CT cv, const T (&w)[NS], int dl) {
     if constexpr (D == 0) {
-      stage_cw<NS, W::YO>(sp, cv, w, dl);
+      if (dl != zeros_at) stage_zero<W::YO>(sp);
+      zeros_at = dl;
+#pragma unroll
+      for (int q = 0; q < NS; ++q) reinterpret_cast<CT*>(sp)[dl + q] = mul2(splat2(w[q]), cv);
+    } else if constexpr (W::BY == 1) {
+      auto at = [&](int p) { return p % W::RS < W::RL && p / W::RS * W::RL + p % W::RS < NS; };
+      using V16 = typename Vec16<T>::type;
+#pragma unroll
+      for (int p = 0; p < W::YN; p += W::R16) {
+        T v[W::R16];
+#pragma unroll
+        for (int i = 0; i < W::R16; ++i) v[i] = at(p + i) ? w[at(p + i) ? (p + i) / W::RS * W::RL + (p + i) % W::RS : 0] : (T)0;
+        *reinterpret_cast<V16*>(sp + W::YO + p) = *reinterpret_cast<const V16*>(v);
+      }
     } else {
       stage_zero<W::YN>(sp + W::YO);
 #pragma unroll
@@ -274,6 +291,8 @@ struct Window<T, 2, NS> {
       }
     }
   }
+  // The slots' memory was used for something else.
+  __device__ __forceinline__ void forget_slot() { zeros_at = -1; }
   __device__ __forceinline__ void add(const T* sp) { add_to(acc, sp); }
   __device__ __forceinline__ void add_to(PT (&sum)[W::RL], const T* sp) {
     const PT cw = *reinterpret_cast<const PT*>(sp + xo);
@@ -358,6 +377,7 @@ struct Window<T, 3, NS> {
 #pragma unroll
       for (int k = 0; k < W::WZ; ++k) acc[i][k] = pair_of((T)0, (T)0);
   }
+  __device__ __forceinline__ void forget_slot() {}
   template <int D>
   static __device__ __forceinline__ void stage(T* sp, CT cv, const T (&w)[NS], int dl) {
     if constexpr (D == 0) {
@@ -476,6 +496,7 @@ __device__ __forceinline__ bool send_sum(Window<T, DIM, NS>& win, const int (&cu
   const bool sent = same(warp);
   __syncthreads();
   if (sent) win.clear();
+  win.forget_slot();
   return !sent && cur[0] >= 0;
 }
 
@@ -647,12 +668,12 @@ __device__ __forceinline__ void spread_window(const PointArgs<T>& a, const cplx_
       }
       T w[NS];
       axis_weights<T, NS>(a, i0[0], xv[0], w);
-      Window<T, DIM, NS>::template stage<0>(my_slot, cv, w, dl[0]);
+      win.template stage<0>(my_slot, cv, w, dl[0]);
       axis_weights<T, NS>(a, i0[1], xv[1], w);
-      Window<T, DIM, NS>::template stage<1>(my_slot, cv, w, dl[1]);
+      win.template stage<1>(my_slot, cv, w, dl[1]);
       if constexpr (DIM == 3) {
         axis_weights<T, NS>(a, i0[2], xv[2], w);
-        Window<T, DIM, NS>::template stage<2>(my_slot, cv, w, dl[2]);
+        win.template stage<2>(my_slot, cv, w, dl[2]);
       }
       // lane j starts a block when its block differs from point j - 1's
       bool differs = false;
