@@ -289,7 +289,8 @@ def secondary_roofs(kernel: str, avg_launch_ms: float, sm_mhz) -> dict | None:
         "shared": {"achieved": wf * 128 / t / 1e9, "peak": smem_peak, "unit": "GB/s",
                    "frac": wf * 128 / t / 1e9 / smem_peak, "wavefronts_per_launch": wf},
         "clock_mhz": float(sm_mhz),
-        "counts_from": "ncu --metrics, one launch per point set (profiles/window_spread.md)",
+        "counts_from": "ncu --metrics, one launch per point set (profiles/"
+                       + ("window_spread.md)" if kernel == "nfx_spread_sorted" else "k_spread_interp_2d_counters.md)"),
     }
 
 

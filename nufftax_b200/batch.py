@@ -5,7 +5,7 @@ precision and dimension).  One `run()` performs, for every problem, a type-1
 transform of its strengths and a type-2 transform of its modes, as
 
     type 1: per-problem bin sorts (concurrent, on side streams) -> ONE
-    persistent spread launch over the work queue of all problems' bin tiles ->
+    persistent spread launch over the work queue of all problems' points ->
     one batched cuFFT per grid-size class -> ONE deconvolve/crop launch;
     type 2: ONE deconvolve/pad launch -> batched cuFFT (both while the points
     sort) -> ONE persistent interp launch once the sorts are done,

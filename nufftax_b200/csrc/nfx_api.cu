@@ -647,6 +647,9 @@ static bool fit_es_poly_uncached(int ns, double beta, double kc, EsPoly& out, do
   return false;
 }
 
+// Fits kept per kernel (ns, beta, kc); a program uses a handful.
+constexpr size_t kKernelsKept = 256;
+
 static bool es_poly(int ns, double beta, double kc, EsPoly& out, double* err = nullptr) {
   static std::mutex mu;
   static std::map<std::tuple<int, double, double>, std::pair<EsPoly, double>> cache;
@@ -654,6 +657,7 @@ static bool es_poly(int ns, double beta, double kc, EsPoly& out, double* err = n
   auto key = std::make_tuple(ns, beta, kc);
   auto it = cache.find(key);
   if (it == cache.end()) {
+    if (cache.size() >= kKernelsKept) cache.clear();
     EsPoly P = {};
     double e = -1.0;
     if (!fit_es_poly_uncached(ns, beta, kc, P, e)) P.deg = 0;
@@ -734,6 +738,7 @@ static void es_polyd(int ns, double beta, double kc, EsPolyD& out) {
   auto key = std::make_tuple(ns, beta, kc);
   auto it = cache.find(key);
   if (it == cache.end()) {
+    if (cache.size() >= kKernelsKept) cache.clear();
     EsPolyD P = {};
     if (!fit_es_polyd(ns, beta, kc, P)) P.deg = 0;
     it = cache.emplace(key, P).first;

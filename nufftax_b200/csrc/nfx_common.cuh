@@ -208,23 +208,6 @@ __device__ __forceinline__ double2 add2(double2 a, double2 b) { return make_doub
 template <typename T> struct PairOf;
 template <> struct PairOf<float> { using type = unsigned long long; };
 template <> struct PairOf<double> { using type = double2; };
-// red_add of a value that is not zero (predicated, no branch).
-__device__ __forceinline__ void red_add_nonzero(float2* addr, float2 v) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.neu.f32 p, %1, 0f00000000;\n setp.neu.or.f32 p, %2, 0f00000000, p;\n"
-      " @p red.global.add.v2.f32 [%0], {%1, %2};\n}" ::"l"(addr), "f"(v.x), "f"(v.y)
-      : "memory");
-}
-__device__ __forceinline__ void red_add_nonzero(double2* addr, double2 v) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.neu.f64 p, %1, 0d0000000000000000;\n"
-      " setp.neu.or.f64 p, %2, 0d0000000000000000, p;\n @p red.global.add.f64 [%0], %1;\n"
-      " @p red.global.add.f64 [%0+8], %2;\n}" ::"l"(addr), "d"(v.x), "d"(v.y)
-      : "memory");
-}
-// c + s * v for a real s and a complex v.
-__device__ __forceinline__ float2 fma_rc(float s, float2 v, float2 c) { return fma2(make_float2(s, s), v, c); }
-__device__ __forceinline__ double2 fma_rc(double s, double2 v, double2 c) { return fma2(make_double2(s, s), v, c); }
 // (s, s) as a complex-typed pair, for a real weight used with many values.
 __device__ __forceinline__ float2 splat2(float s) { return make_float2(s, s); }
 __device__ __forceinline__ double2 splat2(double s) { return make_double2(s, s); }

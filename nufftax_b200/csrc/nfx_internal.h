@@ -148,9 +148,9 @@ constexpr int warps_per_cta(size_t real_bytes, int dim, int ns) { return (real_b
 // Slot layout (2D/3D footprints of at least 32 cells) that the shared-memory
 // budget of a tile counts per staged point: c * w_x (ns complex), then the y
 // weights and (3D) the z weights, padded to the 32 / ns row groups a warp covers
-// and to whole 16-byte chunks.  The window spread's own slots are no larger in
-// total; the budget keeps this form so that the default tiles, and the tiles
-// that are refused, stay what they are.
+// and to whole 16-byte chunks.  The window spread keeps no tile, and its slots are
+// sized by its windows; the budget keeps this form so that the default tiles, and
+// the tiles that are refused, stay what they are.
 // run_slot_reals is 0 when the layout does not apply (1D, small footprints,
 // more than 16 rows a lane).
 __host__ __device__ constexpr int run_groups(int ns) { return 32 / ns; }

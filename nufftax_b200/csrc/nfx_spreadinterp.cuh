@@ -248,14 +248,15 @@ struct Vec16<double> {
 
 namespace nfx {
 
-// Spread of one subproblem, footprints below 32 cells (1D, small ns) or with
-// more than 16 rows a lane (3D, ns >= 9).  Points are staged 32 at a time per
-// warp (weights axis-major), then walked footprint cell by footprint cell with
-// shared-memory atomics on distinct addresses within each instruction.
+// Spread of one subproblem where no window exists (1D; 3D widths from 10).  Points
+// are staged 32 at a time per warp (weights axis-major), then walked footprint cell
+// by footprint cell with shared-memory atomics on distinct addresses within each
+// instruction.
 template <typename T, int DIM, int NS, int NW>
 __device__ __forceinline__ void spread_subproblem_cells(const PointArgs<T>& a, const cplx_t<T>* __restrict__ c,
                                                         cplx_t<T>* __restrict__ fw, int sidx, unsigned char* smem_raw) {
   using CT = cplx_t<T>;
+  static_assert(DIM == 1 || DIM == 3, "2D spreads by windows");
   constexpr int CELLS = Pow<NS, DIM>::value;
   constexpr int SW = NW * 32 + 1;  // staging stride: odd, so both the per-lane writes and
                                    // the per-point reads across q hit distinct banks
@@ -301,7 +302,7 @@ __device__ __forceinline__ void spread_subproblem_cells(const PointArgs<T>& a, c
       }
       __syncwarp();
       const int cnt = min(32, w1 - kb);
-      if constexpr (CELLS >= 32) {
+      if constexpr (DIM == 3) {
         // large footprints: one point at a time, straight to shared memory
         constexpr int R = (CELLS + 31) / 32;
         for (int j = 0; j < cnt; ++j) {
@@ -315,13 +316,7 @@ __device__ __forceinline__ void spread_subproblem_cells(const PointArgs<T>& a, c
               const int kx = q % NS;
               const int ky = (q / NS) % NS;
               const int kz = q / (NS * NS);
-              T w;
-              if (DIM == 1)
-                w = s_w[kx * SW + sj];
-              else if (DIM == 2)
-                w = s_w[(NS + ky) * SW + sj] * s_w[kx * SW + sj];
-              else
-                w = (s_w[(2 * NS + kz) * SW + sj] * s_w[(NS + ky) * SW + sj]) * s_w[kx * SW + sj];
+              const T w = (s_w[(2 * NS + kz) * SW + sj] * s_w[(NS + ky) * SW + sj]) * s_w[kx * SW + sj];
               const int addr = off + kz * plane + ky * row + kx;
               atomicAdd(&s_re[addr], cr * w);
               atomicAdd(&s_im[addr], ci * w);
@@ -333,19 +328,10 @@ __device__ __forceinline__ void spread_subproblem_cells(const PointArgs<T>& a, c
         const int items = cnt * CELLS;
         for (int it = lane; it < items; it += 32) {
           const int j = it / CELLS;
-          const int q = it - j * CELLS;
-          const int kx = q % NS;
-          const int ky = (q / NS) % NS;
-          const int kz = q / (NS * NS);
+          const int kx = it - j * CELLS;
           const int sj = warp * 32 + j;
-          T w;
-          if (DIM == 1)
-            w = s_w[kx * SW + sj];
-          else if (DIM == 2)
-            w = s_w[(NS + ky) * SW + sj] * s_w[kx * SW + sj];
-          else
-            w = (s_w[(2 * NS + kz) * SW + sj] * s_w[(NS + ky) * SW + sj]) * s_w[kx * SW + sj];
-          const int addr = s_off[sj] + kz * plane + ky * row + kx;
+          const T w = s_w[kx * SW + sj];
+          const int addr = s_off[sj] + kx;
           atomicAdd(&s_re[addr], s_cr[sj] * w);
           atomicAdd(&s_im[addr], s_ci[sj] * w);
         }
@@ -748,8 +734,8 @@ __host__ __device__ constexpr int group_lanes() {
   return NS <= 4 ? 4 : (NS <= 8 ? 8 : 16);
 }
 
-// Weight q of one axis: the same arithmetic as axis_weights for that q (cq =
-// the polynomial coefficients of q when the float polynomial is in use).
+// Weight q of one axis: float as axis_weights for that q (cq = the polynomial
+// coefficients of q when the polynomial is in use), double by exp/sqrt.
 template <typename T, int NS>
 __device__ __forceinline__ T axis_weight_q(const PointArgs<T>& a, const float (&cq)[kPolyEvalDeg + 1], int i0, T xs,
                                            int q) {
@@ -1089,8 +1075,8 @@ __global__ void __launch_bounds__(NW * 32, interp_min_ctas<T, DIM, NS, MODE>()) 
 // ---------------------------------------------------------------------------
 // Batched launches: many problems (own points, grid, tiling and sort) in one
 // persistent launch.  `items` is a device table; `sub_prefix[p]` is the number
-// of subproblems of problems < p (k_batch_prefix), so the CTAs walk one global
-// work queue of (problem, bin tile) items.
+// of work items of problems < p (k_batch_prefix; slices of the sorted points or
+// subproblems), so the CTAs walk one global work queue of (problem, item) pairs.
 // ---------------------------------------------------------------------------
 template <typename T>
 struct BatchItem {

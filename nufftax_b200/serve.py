@@ -6,8 +6,8 @@ estimates fit the HBM budget (looking past a head request that does not fit, so
 small requests are not blocked behind a large one).  Admitted small type-1/2
 requests that share a dimension, precision and eps form a WAVE: one library call
 (nfx_wave) enqueues all of them on one slot's stream with one persistent spread
-launch over the bin tiles of every type-1 problem, one persistent interpolation
-over those of every type-2 problem and one launch each for their deconvolution
+launch over the points of every type-1 problem, one persistent interpolation over
+the bin tiles of every type-2 problem and one launch each for their deconvolution
 passes.  Larger requests, type 3 and requests on shared points run alone on a
 slot's stream.  Slots overlap on the device; completion is detected with CUDA
 events and releases the slot and the memory.  Between requests the server keeps

@@ -3,8 +3,9 @@ exp/sqrt) against extended precision.
 
 One point of unit strength spread on its own 1D grid gives the weights
 themselves.  Bound: the fit is accepted within 4e-16 of each weight's largest
-value (at most 1), the edge weights are below 1e-3 with a relative error of a few
-beta roundings, so 6e-16 absolute."""
+value (at most 1); the edge weights by exp/sqrt are off by the rounding of their
+exponent, beta (sqrt(..) - 1), relative to the weight: 0.30 at width 4 (beta 9: about
+1.1e-15 of it), 0.029 at 6, 1.8e-3 at 8 and less beyond.  So 6e-16 absolute."""
 
 import numpy as np
 import pytest
