@@ -517,97 +517,19 @@ __device__ __forceinline__ int win_group_keys(const PointArgs<T>& a, int item) {
   return lane < 2 ? a.s.keys[lane == 0 ? k : k + n - 1] : 0;
 }
 
-// One work item: `a.win_part` consecutive points of the sorted order (of one or
-// several bins); ahead: its win_group_keys (ungrouped).  The CTA groups them by block,
-// then every warp takes a contiguous slice of the grouped list 32 points at a time:
-// each lane stages one point, and the warp adds the 32 one after another, flushing
-// the window whenever the block changes.  The next 32 points are fetched while the
-// current ones are added.
-// A crowded item's points all lie in one block; its warps send one window.  Where a
-// block's points are contiguous, one item of a group of `a.win_group` whose points
-// share a block takes the whole group and the others nothing; which one rotates
-// with the group's place in the grid-stride order, so that each CTA gets its share.
+// The points k0 .. k0 + n - 1 of an item, in the order of `list` (nullptr: as they
+// are), each warp a slice; one_block: the item is crowded.
 template <typename T, int DIM, int NS, int NW>
-__device__ __forceinline__ void spread_window(const PointArgs<T>& a, const cplx_t<T>* __restrict__ c,
-                                              cplx_t<T>* __restrict__ fw, int item, int ahead,
-                                              unsigned char* smem_raw) {
+__device__ __forceinline__ void spread_slices(const PointArgs<T>& a, const cplx_t<T>* __restrict__ c,
+                                              cplx_t<T>* __restrict__ fw, int k0, int n, const unsigned short* list,
+                                              bool one_block, T* s_slots) {
   using CT = cplx_t<T>;
   using W = WinShape<T, DIM, NS>;
-  constexpr int NT = NW * 32;
-  constexpr int PER = (kWinRound + NT - 1) / NT;  // most points of an item per thread
-  __shared__ int s_warp[32];
   const Geom& g = a.g;
-  int k0 = item * a.win_part;
-  int n = (int)min((int64_t)a.win_part, a.M - k0);
-  bool one_block = false;
-  if constexpr (!W::GROUP) {  // a block's points are contiguous: the ends decide
-    one_block = a.win_group > 0 && same_block<T, DIM, NS>(a, __shfl_sync(0xffffffffu, ahead, 0),
-                                                          __shfl_sync(0xffffffffu, ahead, 1));
-    if (one_block) {
-      k0 = win_group_points(a, item, n);
-      const unsigned members = (unsigned)((n + a.win_part - 1) / a.win_part);
-      if (item % a.win_group != (int)((unsigned)item / gridDim.x % members)) return;
-    }
-  }
-  T* s_slots = reinterpret_cast<T*>(smem_raw);
-  int* s_cnt = reinterpret_cast<int*>(s_slots + NT * W::SLOT);  // per block: points, then its list start
-  unsigned short* s_list = reinterpret_cast<unsigned short*>(s_cnt + win_blocks(DIM));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   T* my_slot = s_slots + (warp * 32 + lane) * W::SLOT;
   const T* warp_slots = s_slots + warp * 32 * W::SLOT;
-  // ---- group the points by block: bins in order, blocks within a bin ----
-  bool listed = false;
-  if constexpr (W::GROUP) {
-    const int per_bin = key_block<T, DIM, NS>(g, g.tile[0] * g.tile[1] * g.tile[2] - 1) + 1;  // blocks
-    const int bin0 = a.s.keys[k0] >> a.s.cbits;
-    const int64_t span = (int64_t)((a.s.keys[k0 + n - 1] >> a.s.cbits) - bin0 + 1) * per_bin;
-    // more: sparse points, few of them share a block
-    listed = span <= win_blocks(DIM) && span >= 1;
-    if (listed) {
-      const int nblk = (int)span;
-      const int cmask = (1 << a.s.cbits) - 1;
-      for (int i = threadIdx.x; i < nblk; i += NT) s_cnt[i] = 0;
-      int key[PER], rank[PER];
-#pragma unroll
-      for (int i = 0; i < PER; ++i) {
-        const int j = i * NT + threadIdx.x;
-        key[i] = j < n ? a.s.keys[k0 + j] : -1;
-      }
-      __syncthreads();
-#pragma unroll
-      for (int i = 0; i < PER; ++i) {
-        if (key[i] >= 0) {
-          const int blk = ((key[i] >> a.s.cbits) - bin0) * per_bin + key_block<T, DIM, NS>(g, key[i] & cmask);
-          key[i] = min(max(blk, 0), nblk - 1);  // keys of a sound sort are in range
-          rank[i] = atomicAdd(&s_cnt[key[i]], 1);
-        }
-      }
-      __syncthreads();
-      const int per = (nblk + NT - 1) / NT;
-      const int i0 = min((int)threadIdx.x * per, nblk), i1 = min(i0 + per, nblk);
-      int sum = 0, total;
-      for (int i = i0; i < i1; ++i) sum += s_cnt[i];
-      int run = block_exclusive_scan(sum, s_warp, total);
-      for (int i = i0; i < i1; ++i) {
-        const int v = s_cnt[i];
-        s_cnt[i] = run;
-        run += v;
-      }
-      __syncthreads();
-      bool first = true;  // whether the thread's points lie in the first block that has any
-#pragma unroll
-      for (int i = 0; i < PER; ++i) {
-        if (key[i] >= 0) {
-          const int at = s_cnt[key[i]];
-          first = first && at == 0;
-          s_list[at + rank[i]] = (unsigned short)(i * NT + threadIdx.x);
-        }
-      }
-      one_block = __syncthreads_and(first) && a.win_group > 0;
-    }
-  }
-  // ---- the warp's slice of the list, per transform ----
-  auto list_at = [&](int i) { return W::GROUP && listed ? (int)s_list[i] : i; };
+  auto list_at = [&](int i) { return W::GROUP && list != nullptr ? (int)list[i] : i; };
   const int p0 = (int)((int64_t)n * warp / NW);  // slices differ by at most one point
   const int p1 = (int)((int64_t)n * (warp + 1) / NW);
   Window<T, DIM, NS> win(lane);
@@ -703,6 +625,110 @@ __device__ __forceinline__ void spread_window(const PointArgs<T>& a, const cplx_
     bool open = cur[0] >= 0;
     if (one_block) open = send_sum<T, DIM, NS, NW>(win, cur, g, s_slots, warp, lane, out);
     if (open) win.flush(g, cur[0], cur[1], cur[2], lane, out);
+  }
+}
+
+// A crowded 3D item, by itself: inlined beside the ordinary one, its sum over the
+// warps cost that one's loop 200 bytes of spills (8M points on 256^3 1721 -> 1818 us).
+template <typename T, int DIM, int NS, int NW>
+__device__ __noinline__ void spread_crowded(const PointArgs<T>& a, const cplx_t<T>* __restrict__ c,
+                                            cplx_t<T>* __restrict__ fw, int k0, int n) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  spread_slices<T, DIM, NS, NW>(a, c, fw, k0, n, nullptr, true, reinterpret_cast<T*>(smem_raw));
+}
+
+// One work item: `a.win_part` consecutive points of the sorted order (of one or
+// several bins); ahead: its win_group_keys (ungrouped).  The CTA groups them by block,
+// then every warp takes a contiguous slice of the grouped list 32 points at a time:
+// each lane stages one point, and the warp adds the 32 one after another, flushing
+// the window whenever the block changes.  The next 32 points are fetched while the
+// current ones are added.
+// A crowded item's points all lie in one block; its warps send one window.  Where a
+// block's points are contiguous, one item of a group of `a.win_group` whose points
+// share a block takes the whole group and the others nothing; which one rotates
+// with the group's place in the grid-stride order, so that each CTA gets its share.
+template <typename T, int DIM, int NS, int NW>
+__device__ __forceinline__ void spread_window(const PointArgs<T>& a, const cplx_t<T>* __restrict__ c,
+                                              cplx_t<T>* __restrict__ fw, int item, int ahead,
+                                              unsigned char* smem_raw) {
+  using W = WinShape<T, DIM, NS>;
+  constexpr int NT = NW * 32;
+  constexpr int PER = (kWinRound + NT - 1) / NT;  // most points of an item per thread
+  __shared__ int s_warp[32];
+  const Geom& g = a.g;
+  int k0 = item * a.win_part;
+  int n = (int)min((int64_t)a.win_part, a.M - k0);
+  bool one_block = false;
+  if constexpr (!W::GROUP) {  // a block's points are contiguous: the ends decide
+    one_block = a.win_group > 0 && same_block<T, DIM, NS>(a, __shfl_sync(0xffffffffu, ahead, 0),
+                                                          __shfl_sync(0xffffffffu, ahead, 1));
+    if (one_block) {
+      k0 = win_group_points(a, item, n);
+      const unsigned members = (unsigned)((n + a.win_part - 1) / a.win_part);
+      if (item % a.win_group != (int)((unsigned)item / gridDim.x % members)) return;
+    }
+  }
+  T* s_slots = reinterpret_cast<T*>(smem_raw);
+  int* s_cnt = reinterpret_cast<int*>(s_slots + NT * W::SLOT);  // per block: points, then its list start
+  unsigned short* s_list = reinterpret_cast<unsigned short*>(s_cnt + win_blocks(DIM));
+  // ---- group the points by block: bins in order, blocks within a bin ----
+  bool listed = false;
+  if constexpr (W::GROUP) {
+    const int per_bin = key_block<T, DIM, NS>(g, g.tile[0] * g.tile[1] * g.tile[2] - 1) + 1;  // blocks
+    const int bin0 = a.s.keys[k0] >> a.s.cbits;
+    const int64_t span = (int64_t)((a.s.keys[k0 + n - 1] >> a.s.cbits) - bin0 + 1) * per_bin;
+    // more: sparse points, few of them share a block
+    listed = span <= win_blocks(DIM) && span >= 1;
+    if (listed) {
+      const int nblk = (int)span;
+      const int cmask = (1 << a.s.cbits) - 1;
+      for (int i = threadIdx.x; i < nblk; i += NT) s_cnt[i] = 0;
+      int key[PER], rank[PER];
+#pragma unroll
+      for (int i = 0; i < PER; ++i) {
+        const int j = i * NT + threadIdx.x;
+        key[i] = j < n ? a.s.keys[k0 + j] : -1;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < PER; ++i) {
+        if (key[i] >= 0) {
+          const int blk = ((key[i] >> a.s.cbits) - bin0) * per_bin + key_block<T, DIM, NS>(g, key[i] & cmask);
+          key[i] = min(max(blk, 0), nblk - 1);  // keys of a sound sort are in range
+          rank[i] = atomicAdd(&s_cnt[key[i]], 1);
+        }
+      }
+      __syncthreads();
+      const int per = (nblk + NT - 1) / NT;
+      const int i0 = min((int)threadIdx.x * per, nblk), i1 = min(i0 + per, nblk);
+      int sum = 0, total;
+      for (int i = i0; i < i1; ++i) sum += s_cnt[i];
+      int run = block_exclusive_scan(sum, s_warp, total);
+      for (int i = i0; i < i1; ++i) {
+        const int v = s_cnt[i];
+        s_cnt[i] = run;
+        run += v;
+      }
+      __syncthreads();
+      bool first = true;  // whether the thread's points lie in the first block that has any
+#pragma unroll
+      for (int i = 0; i < PER; ++i) {
+        if (key[i] >= 0) {
+          const int at = s_cnt[key[i]];
+          first = first && at == 0;
+          s_list[at + rank[i]] = (unsigned short)(i * NT + threadIdx.x);
+        }
+      }
+      one_block = __syncthreads_and(first) && a.win_group > 0;
+    }
+  }
+  if constexpr (DIM == 3) {
+    if (one_block)
+      spread_crowded<T, DIM, NS, NW>(a, c, fw, k0, n);
+    else
+      spread_slices<T, DIM, NS, NW>(a, c, fw, k0, n, listed ? s_list : nullptr, false, s_slots);
+  } else {
+    spread_slices<T, DIM, NS, NW>(a, c, fw, k0, n, listed ? s_list : nullptr, one_block, s_slots);
   }
   if constexpr (W::GROUP) __syncthreads();  // the list and counts are free for the next item
 }
