@@ -66,7 +66,9 @@ def on_device(device: torch.device):
 def plain(t: torch.Tensor) -> torch.Tensor:
     """t as its memory should read for a kernel: contiguous, and no lazy conjugate or
     negative view (whose memory holds other values than the tensor stands for)."""
-    return t.resolve_conj().resolve_neg().contiguous()
+    if t.is_conj() or t.is_neg():
+        t = t.resolve_conj().resolve_neg()
+    return t.contiguous()
 
 
 def ptr(t: torch.Tensor | None):
@@ -405,7 +407,9 @@ class TransformPlan:
         them, or the stream captures (a captured FFT takes its own work area)."""
         if recording(*names):
             return True
-        with on_device(self.device):
+        if torch._C._cuda_getDevice() == self.device.index:
+            return torch.cuda.is_current_stream_capturing()
+        with torch.cuda.device(self.device):
             return torch.cuda.is_current_stream_capturing()
 
     def type1(self, ps: PointSort, c: torch.Tensor, sign: int) -> torch.Tensor:
