@@ -259,8 +259,8 @@ ALG_BYTES = {
 # fractions of the issue and shared-memory roofs, the ones that bind these
 # kernels (HBM runs at a few percent of peak).
 MEASURED_COUNTERS = {
-    "nfx_spread_sorted": {"radial": {"dram": 17.28e6, "inst": 25.26e6, "smem_wf": 4.09e6},
-                          "clustered": {"dram": 85.13e6, "inst": 89.16e6, "smem_wf": 26.74e6}},
+    "nfx_spread_sorted": {"radial": {"dram": 17.44e6, "inst": 25.62e6, "smem_wf": 4.26e6},
+                          "clustered": {"dram": 85.34e6, "inst": 87.60e6, "smem_wf": 25.76e6}},
     "nfx_interp_sorted": {"radial": {"dram": 13.53e6, "inst": 7.31e6, "smem_wf": 3.71e6},
                           "clustered": {"dram": 102.01e6, "inst": 43.48e6, "smem_wf": 10.11e6}},
 }

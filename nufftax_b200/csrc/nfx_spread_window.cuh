@@ -25,16 +25,17 @@
 // so each CTA first groups its item's points by block with a counting sort of
 // 16-bit indices in shared memory (two passes over the sorted keys).  2D
 // complex64: segments of 8x1 cells, which are contiguous, so nothing is grouped
-// (8x4 blocks measured 227 us instead of 146 on 4M clustered points: grouping
+// (8x4 blocks measured 227 us on 4M clustered points, segments 157: grouping
 // and the wider window cost more than the reds they save).  2D complex128:
 // blocks, since a wide kernel's window is all reds.
 //
 // What bounds it now (sorted points, L2 flushed before each call; before = the
 // shared-memory tile spreads it replaces): 3D 8M points on 256^3, ns 8: 3645 ->
-// 1725 us (FMA pipe 51 %, issue 54 %); 1M on 192x225x256: 781 -> 505 us (reds,
-// L2 57 %); 2D 524 k radial on 1024^2, ns 8: 91 -> 52 us, 4M clustered 163 -> 146
-// us (staging: issue 63 %, shared memory 87 %); 2D complex128 ns 14, 200 k
-// points: 412 -> 97 us, 79 with polynomial weights (reds, L2 59 %).
+// 1700 us (FMA pipe 52 %, issue 51 %); 1M on 192x225x256: 781 -> 509 us (reds);
+// 2D 524 k radial on 1024^2, ns 8: 91 -> 54 us; complex128 ns 14, 200 k points: 412
+// -> 79 us (reds).  Dense 2D complex64 sets are bound by their staging (issue 65 %,
+// shared memory) and gain little or lose: 4M clustered points 163 -> 157 us, 8M 242
+// -> 261.
 #pragma once
 
 #include <type_traits>
@@ -109,7 +110,7 @@ struct WinShape<T, 1, NS> {
 };
 
 // Warps per CTA of the spread (the window of 44 complex64 cells a lane needs
-// about 160 registers to run without spills).
+// 168 registers, 68 bytes of them spilled).
 template <typename T, int DIM, int NS>
 constexpr int win_warps() {
   return sizeof(T) == 4 && DIM == 3 && NS == 8 ? 6 : warps_per_cta(sizeof(T), DIM, NS);
